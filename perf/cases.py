@@ -93,8 +93,11 @@ def draw(rng):
         n = mx << level
         room = 1.5e11 / (n * n * OPS[eq])
         steps = max(3, min(int(math.exp(rng.uniform(math.log(7), math.log(200)))), int(room)))
-        walls = eq != "advection" and rng.random() < 0.5
-        return _case(None, kind, eq, mx, level, level, steps, precision, version, rng.choice((1, 2, 3, 4, 4)), walls,
+        # the quadrants' inflow tears away from a wall, and superbee sharpens the
+        # systems' waves into noise over thousands of steps
+        walls = eq == "swe" and rng.random() < 0.5
+        limiter = rng.choice((1, 2, 3, 4, 4) if eq == "advection" else (1, 3, 4, 4))
+        return _case(None, kind, eq, mx, level, level, steps, precision, version, limiter, walls,
                      kind == "level" or rng.random() < 0.3)
     eq = rng.choice(("swe", "swe", "euler", "geoclaw", "filament"))
     if kind == "run":
@@ -118,9 +121,10 @@ def _n(case):
 
 
 def _dt(case):
-    """A fixed step of CFL 0.5 to 0.9 on the coarsest level of the mesh."""
+    """A fixed step of CFL 0.3 to 0.9 on the coarsest level of the mesh, with room for
+    what the state may become after many passes."""
     n = case["mx"] << case["minlevel"]
-    return {"advection": 0.9, "swe": 0.4, "euler": 0.3, "geoclaw": 0.5, "filament": 0.08}[case["equation"]] / n
+    return {"advection": 0.9, "swe": 0.3, "euler": 0.2, "geoclaw": 0.5, "filament": 0.08}[case["equation"]] / n
 
 
 def _options(case, seed):
