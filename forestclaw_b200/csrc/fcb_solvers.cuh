@@ -10,6 +10,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fcb_arith.cuh"
+
 namespace fcb {
 
 template <typename T>
@@ -115,6 +117,16 @@ struct AuxLayout<AdvectionManifoldSolver<W_, V5_>> {
 // ---------------------------------------------------------------------------
 // V5: clawpack5_rpn2.f90, clawpack5_rpt2.f90 (a1, a3 scaled by 0.5/a instead
 // of divided by 2a; the Roe averages clawpack5_rpt2 recomputes equal rpn2's).
+//
+// A Riemann problem is solved in three parts, so that a kernel can keep the Roe
+// averages and wave strengths (roe) and form the waves (waves) or the fluctuations
+// (fluct) when it needs them.  Each takes the common case without branches: the
+// quotients with one divisor share its reciprocal (fcb_arith.cuh), and the entropy
+// fix, which needs the speeds of the states left and right of the middle waves only
+// for their signs, decides those by comparing squares (u > c exactly when u > 0 and
+// (hu)^2 > g h^3) with a margin of 0.1 %, far above rounding.  A transonic wave, a
+// comparison inside the margin and operands near underflow take the reference's
+// formulas as they stand (exact_*).
 template <typename R, bool V5_ = false>
 struct SweRoeT {
     using Real = R;
@@ -122,21 +134,32 @@ struct SweRoeT {
     static constexpr bool FWAVE = false;
     static constexpr int M = 3;
     static constexpr int W = 3;
-    struct Roe { R u, v, a; };
+    // y: what divides by 2a (clawpack 5: 0.5/a; 0: use the operator); a1..a3: wave strengths
+    struct Roe { R u, v, a, y, a1, a2, a3; };
     // Quantities of one cell that every Riemann problem it takes part in (two
     // x- and two y-interfaces) evaluates with the same operations on the same
-    // operands: sqrt(h), hu/sqrt(h), hv/sqrt(h), hu/h, hv/h, sqrt(g h).  The
-    // step kernels compute them once per cell; the values are bit-identical.
-    struct Cell { R sq, rq[2], vel[2], c; };
-    static constexpr int NC = 6;
+    // operands: sqrt(h), hu/sqrt(h), hv/sqrt(h); and g h^3 for the sign tests.
+    // The step kernels compute them once per cell; the values are bit-identical.
+    struct Cell { R sq, rq[2], gh3; };
+    static constexpr int NC = 4;
+    // wave components that are not zero by construction (component order: depth,
+    // normal and transverse momentum): the middle wave is a shear
+    static constexpr int NWV = 7;
+    __host__ __device__ static constexpr bool nz(int mw, int rel) { return mw != 1 || rel == 2; }
     R grav, gamma, gamma1, drytol;  // drytol: GeoClaw only
     __device__ __forceinline__ void prep(const R* q, Cell& k) const {
-        k.sq = sqrt(q[0]);
-        k.rq[0] = q[1] / k.sq;
-        k.rq[1] = q[2] / k.sq;
-        k.vel[0] = q[1] / q[0];
-        k.vel[1] = q[2] / q[0];
-        k.c = sqrt(grav * q[0]);
+        bool ok = true;
+        k.sq = sqrt_ok(q[0], ok);
+        const Dv<R> d(k.sq, ok);
+        k.rq[0] = d(q[1], ok);
+        k.rq[1] = d(q[2], ok);
+        if (!ok) {
+            seldom();
+            k.sq = sqrt(q[0]);
+            k.rq[0] = q[1] / k.sq;
+            k.rq[1] = q[2] / k.sq;
+        }
+        k.gh3 = grav * q[0] * q[0] * q[0];
     }
     __device__ __forceinline__ void rpn2(int ixy, const R* qL, const R* qR, R speed,
                                          R (*wave)[M], R* s, R* amdq, R* apdq,
@@ -149,75 +172,166 @@ struct SweRoeT {
     __device__ __forceinline__ void rpn2c(int ixy, const R* qL, const R* qR, const Cell& cl, const Cell& cr,
                                           R /*speed*/, R (*wave)[M], R* s, R* amdq, R* apdq,
                                           Roe& rr) const {
+        roe(ixy, qL, qR, cl, cr, rr);
+        waves(ixy, rr, wave, s);
+        fluct(ixy, qL, qR, cl, cr, wave, s, amdq, apdq);
+    }
+    __device__ __forceinline__ void roe(int ixy, const R* qL, const R* qR, const Cell& cl, const Cell& cr,
+                                        Roe& rr) const {
         const int mu = (ixy == 1) ? 1 : 2;
         const int mv = (ixy == 1) ? 2 : 1;
+        bool ok = true;
         const R h = (qL[0] + qR[0]) / R(2.0);
-        const R hsq2 = cl.sq + cr.sq;                       // sqrt(qL(1)) + sqrt(qR(1))
-        const R u = (cl.rq[mu - 1] + cr.rq[mu - 1]) / hsq2;  // (qL(mu)/hsqrtl + qR(mu)/hsqrtr)/hsq2
-        const R v = (cl.rq[mv - 1] + cr.rq[mv - 1]) / hsq2;
-        const R a = sqrt(grav * h);
+        const Dv<R> dh(cl.sq + cr.sq, ok);                // sqrt(qL(1)) + sqrt(qR(1))
+        const R u = dh(cl.rq[mu - 1] + cr.rq[mu - 1], ok);  // (qL(mu)/hsqrtl + qR(mu)/hsqrtr)/hsq2
+        const R v = dh(cl.rq[mv - 1] + cr.rq[mv - 1], ok);
+        const R a = sqrt_ok(grav * h, ok);
+        const Dv<R> da(V5 ? a : R(2.0) * a, ok);
         rr.u = u; rr.v = v; rr.a = a;
+        rr.y = V5 ? da.scaled(R(0.5)) : da.y;
         const R d1 = qR[0] - qL[0];
         const R d2 = qR[mu] - qL[mu];
         const R d3 = qR[mv] - qL[mv];
-        const R a1 = V5 ? ((u + a) * d1 - d2) * (R(0.5) / a) : ((u + a) * d1 - d2) / (R(2.0) * a);
-        const R a2 = -(v * d1) + d3;
-        const R a3 = V5 ? (-((u - a) * d1) + d2) * (R(0.5) / a) : (-((u - a) * d1) + d2) / (R(2.0) * a);
-        wave[0][0] = a1; wave[0][mu] = a1 * (u - a); wave[0][mv] = a1 * v; s[0] = u - a;
-        wave[1][0] = R(0.0); wave[1][mu] = R(0.0); wave[1][mv] = a2; s[1] = u;
-        wave[2][0] = a3; wave[2][mu] = a3 * (u + a); wave[2][mv] = a3 * v; s[2] = u + a;
-        // entropy fix
-        R am[3];
-        {
-            const R s0 = cl.vel[mu - 1] - cl.c;  // qL(mu)/him1 - sqrt(g*him1)
-            R sfract;
-            if (s0 > R(0.0) && s[0] > R(0.0)) {
-                am[0] = am[1] = am[2] = R(0.0);
-                goto done;
-            }
-            {
-                const R h1 = qL[0] + wave[0][0];
-                const R hu1 = qL[mu] + wave[0][mu];
-                const R s1 = hu1 / h1 - sqrt(grav * h1);
-                if (s0 < R(0.0) && s1 > R(0.0)) sfract = s0 * ((s1 - s[0]) / (s1 - s0));
-                else if (s[0] < R(0.0)) sfract = s[0];
-                else sfract = R(0.0);
-#pragma unroll
-                for (int m = 0; m < 3; ++m) am[m] = sfract * wave[0][m];
-            }
-            if (s[1] > R(0.0)) goto done;
-#pragma unroll
-            for (int m = 0; m < 3; ++m) am[m] = am[m] + s[1] * wave[1][m];
-            {
-                const R s03 = cr.vel[mu - 1] + cr.c;  // qR(mu)/hi + sqrt(g*hi)
-                const R h3 = qR[0] - wave[2][0];
-                const R hu3 = qR[mu] - wave[2][mu];
-                const R s3 = hu3 / h3 + sqrt(grav * h3);
-                if (s3 < R(0.0) && s03 > R(0.0)) sfract = s3 * ((s03 - s[2]) / (s03 - s3));
-                else if (s[2] < R(0.0)) sfract = s[2];
-                else goto done;
-#pragma unroll
-                for (int m = 0; m < 3; ++m) am[m] = am[m] + sfract * wave[2][m];
-            }
+        rr.a1 = V5 ? ((u + a) * d1 - d2) * rr.y : da((u + a) * d1 - d2, ok);
+        rr.a2 = -(v * d1) + d3;
+        rr.a3 = V5 ? (-((u - a) * d1) + d2) * rr.y : da(-((u - a) * d1) + d2, ok);
+        if (!ok) {
+            seldom();
+            const R l[3] = {qL[0], qL[mu], qL[mv]}, r[3] = {qR[0], qR[mu], qR[mv]};
+            rr = exact_roe(l[0], l[1], l[2], r[0], r[1], r[2], grav);
         }
-    done:
+    }
+    __device__ __forceinline__ void speeds(const Roe& rr, R* s) const {
+        s[0] = rr.u - rr.a;
+        s[1] = rr.u;
+        s[2] = rr.u + rr.a;
+    }
+    __device__ __forceinline__ void waves(int ixy, const Roe& rr, R (*wave)[M], R* s) const {
+        const int mu = (ixy == 1) ? 1 : 2;
+        const int mv = (ixy == 1) ? 2 : 1;
+        speeds(rr, s);
+        wave[0][0] = rr.a1; wave[0][mu] = rr.a1 * s[0]; wave[0][mv] = rr.a1 * rr.v;
+        wave[1][0] = R(0.0); wave[1][mu] = R(0.0); wave[1][mv] = rr.a2;
+        wave[2][0] = rr.a3; wave[2][mu] = rr.a3 * s[2]; wave[2][mv] = rr.a3 * rr.v;
+    }
+    __device__ __forceinline__ void fluct(int ixy, const R* qL, const R* qR, const Cell& cl, const Cell& cr,
+                                          const R (*wave)[M], const R* s, R* amdq, R* apdq) const {
+        const int mu = (ixy == 1) ? 1 : 2;
+        const int mv = (ixy == 1) ? 2 : 1;
+        // entropy fix: left of the first wave the speed s0 = u - c of qL, right of it s1
+        const R g = grav, lo = R(0.999), hi = R(1.001);
+        const R mL = qL[mu], mL2 = mL * mL;
+        const bool supL = mL > R(0.0) && mL2 > hi * cl.gh3;   // s0 > 0
+        const bool subL = mL <= R(0.0) || mL2 < lo * cl.gh3;  // s0 < 0
+        const R h1 = qL[0] + wave[0][0], hu1 = mL + wave[0][mu];
+        const bool sub1 = h1 > R(0.0) && (hu1 <= R(0.0) || hu1 * hu1 < lo * (g * h1 * h1 * h1));  // s1 < 0
+        // right of the third wave s03 = u + c of qR, left of it s3
+        const bool right = s[1] <= R(0.0);
+        const R mR = qR[mu];
+        const bool supR = mR < R(0.0) && mR * mR > hi * cr.gh3;  // s03 < 0
+        const R h3 = qR[0] - wave[2][0], hu3 = mR - wave[2][mu];
+        const bool sub3 = h3 > R(0.0) && (hu3 >= R(0.0) || hu3 * hu3 < lo * (g * h3 * h3 * h3));  // s3 > 0
+        const bool ok = (qL[0] > R(0.0)) & (supL | (subL & sub1)) & ((s[1] > R(0.0)) | (right & (sub3 | supR)));
+        const R k0 = s[0] < R(0.0) ? s[0] : R(0.0);
+        const R k1 = right ? s[1] : R(0.0);
+        const R k2 = right && s[2] < R(0.0) ? s[2] : R(0.0);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            R am = k0 * wave[0][m];
+            if (m == mv) am = am + k1 * wave[1][m];  // the other components are zero
+            amdq[m] = am + k2 * wave[2][m];
+        }
+        if (!ok) {
+            seldom();
+            const Fluct e = exact_fluct(qL[0], mL, qL[mv], qR[0], mR, qR[mv], grav, wave[0][0], wave[1][mv], wave[2][0],
+                                        wave[0][mu], wave[0][mv], wave[2][mu], wave[2][mv], s[0], s[1], s[2]);
+            amdq[0] = e.am[0];
+            amdq[mu] = e.am[1];
+            amdq[mv] = e.am[2];
+        }
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
             R df = s[0] * wave[0][m];
 #pragma unroll
-            for (int mw = 1; mw < W; ++mw) df = df + s[mw] * wave[mw][m];
-            amdq[m] = am[m];
-            apdq[m] = df - am[m];
+            for (int mw = 1; mw < W; ++mw)
+                if (nz(mw, m == mv ? 2 : m == 0 ? 0 : 1)) df = df + s[mw] * wave[mw][m];
+            apdq[m] = df - amdq[m];
         }
+    }
+    // The reference's formulas, components in the order depth, normal, transverse.
+    static __device__ __forceinline__ Roe exact_roe(R l0, R l1, R l2, R r0, R r1, R r2, R grav) {
+        const R sl = sqrt(l0), sr = sqrt(r0);
+        const R h = (l0 + r0) / R(2.0);
+        const R hsq2 = sl + sr;
+        Roe rr;
+        const R u = rr.u = (l1 / sl + r1 / sr) / hsq2;
+        const R v = rr.v = (l2 / sl + r2 / sr) / hsq2;
+        const R a = rr.a = sqrt(grav * h);
+        const R d1 = r0 - l0, d2 = r1 - l1, d3 = r2 - l2;
+        rr.a1 = V5 ? ((u + a) * d1 - d2) * (R(0.5) / a) : ((u + a) * d1 - d2) / (R(2.0) * a);
+        rr.a2 = -(v * d1) + d3;
+        rr.a3 = V5 ? (-((u - a) * d1) + d2) * (R(0.5) / a) : (-((u - a) * d1) + d2) / (R(2.0) * a);
+        bool in = true;
+        const Dv<R> da(V5 ? a : R(2.0) * a, in);
+        rr.y = V5 ? R(0.5) / a : in ? da.y : R(0.0);
+        return rr;
+    }
+    struct Fluct { R am[3]; };
+    static __device__ __forceinline__ Fluct exact_fluct(R l0, R l1, R l2, R r0, R r1, R r2, R grav, R w00, R w12, R w20,
+                                                     R w01, R w02, R w21, R w22, R sA, R sB, R sC) {
+        Fluct e;
+        R* am = e.am;
+        const R s0 = l1 / l0 - sqrt(grav * l0);
+        R sfract;
+        if (s0 > R(0.0) && sA > R(0.0)) {
+            am[0] = am[1] = am[2] = R(0.0);
+            return e;
+        }
+        const R h1 = l0 + w00;
+        const R hu1 = l1 + w01;
+        const R s1 = hu1 / h1 - sqrt(grav * h1);
+        if (s0 < R(0.0) && s1 > R(0.0)) sfract = s0 * ((s1 - sA) / (s1 - s0));
+        else if (sA < R(0.0)) sfract = sA;
+        else sfract = R(0.0);
+        am[0] = sfract * w00;
+        am[1] = sfract * w01;
+        am[2] = sfract * w02;
+        if (sB > R(0.0)) return e;
+        am[2] = am[2] + sB * w12;  // the other components are zero
+        const R s03 = r1 / r0 + sqrt(grav * r0);
+        const R h3 = r0 - w20;
+        const R hu3 = r1 - w21;
+        const R s3 = hu3 / h3 + sqrt(grav * h3);
+        if (s3 < R(0.0) && s03 > R(0.0)) sfract = s3 * ((s03 - sC) / (s03 - s3));
+        else if (sC < R(0.0)) sfract = sC;
+        else return e;
+        am[0] = am[0] + sfract * w20;
+        am[1] = am[1] + sfract * w21;
+        am[2] = am[2] + sfract * w22;
+        return e;
     }
     __device__ __forceinline__ void rpt2(int ixy, const R* asdq, const Roe& rr, R, R,
                                          R* bm, R* bp) const {
         const int mu = (ixy == 1) ? 1 : 2;
         const int mv = (ixy == 1) ? 2 : 1;
         const R u = rr.u, v = rr.v, a = rr.a;
-        const R a1 = V5 ? (R(0.5) / a) * ((v + a) * asdq[0] - asdq[mv]) : ((v + a) * asdq[0] - asdq[mv]) / (2 * a);
+        const R x1 = (v + a) * asdq[0] - asdq[mv], x3 = -((v - a) * asdq[0]) + asdq[mv];
+        R a1, a3;
+        if constexpr (V5) {
+            a1 = rr.y * x1;  // y = 0.5/a
+            a3 = rr.y * x3;
+        } else {
+            bool ok = sizeof(R) == 4 || rr.y != R(0.0);
+            const Dv<R> d(2 * a, rr.y);
+            a1 = d(x1, ok);
+            a3 = d(x3, ok);
+            if (!ok) {
+                seldom();
+                a1 = x1 / (2 * a);
+                a3 = x3 / (2 * a);
+            }
+        }
         const R a2 = asdq[mu] - u * asdq[0];
-        const R a3 = V5 ? (R(0.5) / a) * (-((v - a) * asdq[0]) + asdq[mv]) : (-((v - a) * asdq[0]) + asdq[mv]) / (2 * a);
         R waveb[3][3], sb[3];
         waveb[0][0] = a1; waveb[mu][0] = a1 * u; waveb[mv][0] = a1 * (v - a); sb[0] = v - a;
         waveb[0][1] = R(0.0); waveb[mu][1] = a2; waveb[mv][1] = R(0.0); sb[1] = v;
@@ -227,6 +341,7 @@ struct SweRoeT {
             R m1 = dmin(sb[0], R(0.0)) * waveb[m][0], p1 = dmax(sb[0], R(0.0)) * waveb[m][0];
 #pragma unroll
             for (int mw = 1; mw < 3; ++mw) {
+                if (mw == 1 && m != mu) continue;  // waveb[m][1] is zero
                 m1 = m1 + dmin(sb[mw], R(0.0)) * waveb[m][mw];
                 p1 = p1 + dmax(sb[mw], R(0.0)) * waveb[m][mw];
             }
@@ -249,24 +364,36 @@ struct Euler4RoeT {
     static constexpr bool FWAVE = false;
     static constexpr int M = 4;
     static constexpr int W = 4;
-    struct Roe { R u, v, a, enth, u2v2, g1a2, euv; };
+    // y: what divides by 2a (0: use the operator); a1..a4: wave strengths
+    struct Roe { R u, v, a, enth, g1a2, y, a1, a2, a3, a4; };
     // Quantities of one cell shared by the four Riemann problems it takes part
-    // in: sqrt(rho), rho u/sqrt(rho), rho v/sqrt(rho), (E + p)/sqrt(rho), u, v
-    // and the sound speed sqrt(gamma p/rho).  The entropy fix's pressure sums
-    // the squared momenta in the normal direction's order, which equals p
-    // (addition commutes exactly), so every value is bit-identical.
-    struct Cell { R sq, rq[2], rh, vel[2], c; };
-    static constexpr int NC = 7;
+    // in: sqrt(rho), rho u/sqrt(rho), rho v/sqrt(rho), (E + p)/sqrt(rho); and
+    // gamma p rho for the sign tests.  Every value is bit-identical.
+    struct Cell { R sq, rq[2], rh, gpr; };
+    static constexpr int NC = 5;
+    // wave components that are not zero by construction (density, normal and
+    // transverse momentum, energy): the second wave is a shear
+    static constexpr int NWV = 14;
+    __host__ __device__ static constexpr bool nz(int mw, int rel) { return mw != 1 || rel >= 2; }
     R grav, gamma, gamma1, drytol;  // drytol: GeoClaw only
     __device__ __forceinline__ void prep(const R* q, Cell& k) const {
-        k.sq = sqrt(q[0]);
-        const R p = gamma1 * (q[3] - R(0.5) * (q[1] * q[1] + q[2] * q[2]) / q[0]);
-        k.rq[0] = q[1] / k.sq;
-        k.rq[1] = q[2] / k.sq;
-        k.rh = (q[3] + p) / k.sq;
-        k.vel[0] = q[1] / q[0];
-        k.vel[1] = q[2] / q[0];
-        k.c = sqrt(gamma * p / q[0]);
+        bool ok = true;
+        k.sq = sqrt_ok(q[0], ok);
+        const Dv<R> dr(q[0], ok), ds(k.sq, ok);
+        const R ke = R(0.5) * (q[1] * q[1] + q[2] * q[2]);
+        R p = gamma1 * (q[3] - dr(ke, ok));
+        k.rq[0] = ds(q[1], ok);
+        k.rq[1] = ds(q[2], ok);
+        k.rh = ds(q[3] + p, ok);
+        if (!ok) {
+            seldom();
+            k.sq = sqrt(q[0]);
+            p = gamma1 * (q[3] - ke / q[0]);
+            k.rq[0] = q[1] / k.sq;
+            k.rq[1] = q[2] / k.sq;
+            k.rh = (q[3] + p) / k.sq;
+        }
+        k.gpr = gamma * p * q[0];
     }
     __device__ __forceinline__ void rpn2(int ixy, const R* qL, const R* qR, R speed,
                                          R (*wave)[M], R* s, R* amdq, R* apdq,
@@ -279,100 +406,208 @@ struct Euler4RoeT {
     __device__ __forceinline__ void rpn2c(int ixy, const R* qL, const R* qR, const Cell& cl, const Cell& cr, R,
                                           R (*wave)[M], R* s, R* amdq, R* apdq,
                                           Roe& rr) const {
+        roe(ixy, qL, qR, cl, cr, rr);
+        waves(ixy, rr, wave, s);
+        fluct(ixy, qL, qR, cl, cr, wave, s, amdq, apdq);
+    }
+    // The three parts of a Riemann problem as the shallow-water solver has them:
+    // u > c exactly when rho u > 0 and (rho u)^2 > gamma p rho.
+    __device__ __forceinline__ void roe(int ixy, const R* qL, const R* qR, const Cell& cl, const Cell& cr,
+                                        Roe& rr) const {
         const int mu = (ixy == 1) ? 1 : 2;
         const int mv = (ixy == 1) ? 2 : 1;
-        const R rhsq2 = cl.sq + cr.sq;
-        const R u = (cl.rq[mu - 1] + cr.rq[mu - 1]) / rhsq2;  // (qL(mu)/rhsqrtl + qR(mu)/rhsqrtr)/rhsq2
-        const R v = (cl.rq[mv - 1] + cr.rq[mv - 1]) / rhsq2;
-        const R enth = (cl.rh + cr.rh) / rhsq2;               // ((qL(4)+pl)/rhsqrtl + (qR(4)+pr)/rhsqrtr)/rhsq2
+        bool ok = true;
+        const Dv<R> dh(cl.sq + cr.sq, ok);
+        const R u = dh(cl.rq[mu - 1] + cr.rq[mu - 1], ok);  // (qL(mu)/rhsqrtl + qR(mu)/rhsqrtr)/rhsq2
+        const R v = dh(cl.rq[mv - 1] + cr.rq[mv - 1], ok);
+        const R enth = dh(cl.rh + cr.rh, ok);               // ((qL(4)+pl)/rhsqrtl + (qR(4)+pr)/rhsqrtr)/rhsq2
         const R u2v2 = u * u + v * v;
         const R a2s = gamma1 * (enth - R(0.5) * u2v2);
-        const R a = sqrt(a2s);
-        const R g1a2 = gamma1 / a2s;
-        const R euv = enth - u2v2;
-        rr.u = u; rr.v = v; rr.a = a; rr.enth = enth; rr.u2v2 = u2v2; rr.g1a2 = g1a2; rr.euv = euv;
+        const R a = sqrt_ok(a2s, ok);
+        const Dv<R> d2s(a2s, ok), da(R(2.0) * a, ok);
+        rr.u = u; rr.v = v; rr.a = a; rr.enth = enth; rr.y = da.y;
+        rr.g1a2 = d2s(gamma1, ok);
         const R d1 = qR[0] - qL[0];
         const R d2 = qR[mu] - qL[mu];
         const R d3 = qR[mv] - qL[mv];
         const R d4 = qR[3] - qL[3];
-        const R a3 = g1a2 * (euv * d1 + u * d2 + v * d3 - d4);
-        const R a2 = d3 - v * d1;
-        const R a4 = (d2 + (a - u) * d1 - a * a3) / (R(2.0) * a);
-        const R a1 = d1 - a3 - a4;
-        wave[0][0] = a1; wave[0][mu] = a1 * (u - a); wave[0][mv] = a1 * v; wave[0][3] = a1 * (enth - u * a);
-        s[0] = u - a;
-        wave[1][0] = R(0.0); wave[1][mu] = R(0.0); wave[1][mv] = a2; wave[1][3] = a2 * v; s[1] = u;
-        wave[2][0] = a3; wave[2][mu] = a3 * u; wave[2][mv] = a3 * v; wave[2][3] = a3 * R(0.5) * u2v2; s[2] = u;
-        wave[3][0] = a4; wave[3][mu] = a4 * (u + a); wave[3][mv] = a4 * v; wave[3][3] = a4 * (enth + u * a);
-        s[3] = u + a;
-        R am[4];
-        {
-            const R s0 = cl.vel[mu - 1] - cl.c;  // qL(mu)/rhoim1 - sqrt(gamma*pim1/rhoim1)
-            R sfract;
-            if (s0 >= R(0.0) && s[0] > R(0.0)) {
-                am[0] = am[1] = am[2] = am[3] = R(0.0);
-                goto done;
-            }
-            {
-                const R rho1 = qL[0] + wave[0][0];
-                const R rhou1 = qL[mu] + wave[0][mu];
-                const R rhov1 = qL[mv] + wave[0][mv];
-                const R en1 = qL[3] + wave[0][3];
-                const R p1 = gamma1 * (en1 - R(0.5) * (rhou1 * rhou1 + rhov1 * rhov1) / rho1);
-                const R c1 = sqrt(gamma * p1 / rho1);
-                const R s1 = rhou1 / rho1 - c1;
-                if (s0 < R(0.0) && s1 > R(0.0)) sfract = s0 * (s1 - s[0]) / (s1 - s0);
-                else if (s[0] < R(0.0)) sfract = s[0];
-                else sfract = R(0.0);
+        rr.a3 = rr.g1a2 * ((enth - u2v2) * d1 + u * d2 + v * d3 - d4);
+        rr.a2 = d3 - v * d1;
+        rr.a4 = da(d2 + (a - u) * d1 - a * rr.a3, ok);
+        rr.a1 = d1 - rr.a3 - rr.a4;
+        if (!ok) {
+            seldom();
+            const R l[4] = {qL[0], qL[mu], qL[mv], qL[3]}, r[4] = {qR[0], qR[mu], qR[mv], qR[3]};
+            // the pressure sums the squared momenta in either order: addition commutes
+            rr = exact_roe(l[0], l[1], l[2], l[3], r[0], r[1], r[2], r[3], gamma1);
+        }
+    }
+    __device__ __forceinline__ void speeds(const Roe& rr, R* s) const {
+        s[0] = rr.u - rr.a;
+        s[1] = s[2] = rr.u;
+        s[3] = rr.u + rr.a;
+    }
+    __device__ __forceinline__ void waves(int ixy, const Roe& rr, R (*wave)[M], R* s) const {
+        const int mu = (ixy == 1) ? 1 : 2;
+        const int mv = (ixy == 1) ? 2 : 1;
+        const R u = rr.u, v = rr.v, ua = u * rr.a, u2v2 = u * u + v * v;
+        speeds(rr, s);
+        wave[0][0] = rr.a1; wave[0][mu] = rr.a1 * s[0]; wave[0][mv] = rr.a1 * v; wave[0][3] = rr.a1 * (rr.enth - ua);
+        wave[1][0] = R(0.0); wave[1][mu] = R(0.0); wave[1][mv] = rr.a2; wave[1][3] = rr.a2 * v;
+        wave[2][0] = rr.a3; wave[2][mu] = rr.a3 * u; wave[2][mv] = rr.a3 * v; wave[2][3] = rr.a3 * R(0.5) * u2v2;
+        wave[3][0] = rr.a4; wave[3][mu] = rr.a4 * s[3]; wave[3][mv] = rr.a4 * v; wave[3][3] = rr.a4 * (rr.enth + ua);
+    }
+    __device__ __forceinline__ void fluct(int ixy, const R* qL, const R* qR, const Cell& cl, const Cell& cr,
+                                          const R (*wave)[M], const R* s, R* amdq, R* apdq) const {
+        const int mu = (ixy == 1) ? 1 : 2;
+        const int mv = (ixy == 1) ? 2 : 1;
+        // entropy fix: left of the first wave the speed s0 = u - c of qL, right of it s1.
+        // The products with the density cancel where the pressure is small against
+        // the energy: such states are left to exact_fluct().
+        const R lo = R(0.999), hi = R(1.001), pmin = sizeof(R) == 8 ? R(1e-8) : R(1e-2);
+        const R mL = qL[mu], mL2 = mL * mL;
+        const bool posL = qL[0] > R(0.0) && cl.gpr > R(0.0), posR = qR[0] > R(0.0) && cr.gpr > R(0.0);
+        const bool supL = posL && mL > R(0.0) && mL2 > hi * cl.gpr;     // s0 > 0
+        const bool subL = posL && (mL <= R(0.0) || mL2 < lo * cl.gpr);  // s0 < 0
+        const R r1 = qL[0] + wave[0][0], m1 = mL + wave[0][mu], t1 = qL[mv] + wave[0][mv];
+        const R e1 = (qL[3] + wave[0][3]) * r1, pr1 = gamma1 * (e1 - R(0.5) * (m1 * m1 + t1 * t1));
+        const bool sub1 = r1 > R(0.0) && pr1 > pmin * e1 && (m1 <= R(0.0) || m1 * m1 < lo * (gamma * pr1));  // s1 < 0
+        // right of the fourth wave s3 = u + c of qR, left of it s2
+        const bool right = s[1] < R(0.0);
+        const R mR = qR[mu];
+        const bool supR = posR && mR < R(0.0) && mR * mR > hi * cr.gpr;  // s3 < 0
+        const R r2 = qR[0] - wave[3][0], m2 = mR - wave[3][mu], t2 = qR[mv] - wave[3][mv];
+        const R e2 = (qR[3] - wave[3][3]) * r2, pr2 = gamma1 * (e2 - R(0.5) * (m2 * m2 + t2 * t2));
+        const bool sub2 = r2 > R(0.0) && pr2 > pmin * e2 && (m2 >= R(0.0) || m2 * m2 < lo * (gamma * pr2));  // s2 > 0
+        const bool ok = (supL | (subL & sub1)) & ((s[1] >= R(0.0)) | (right & (sub2 | supR)));
+        const R k0 = s[0] < R(0.0) ? s[0] : R(0.0);
+        const R k1 = right ? s[1] : R(0.0);
+        const R k3 = right && s[3] < R(0.0) ? s[3] : R(0.0);
 #pragma unroll
-                for (int m = 0; m < 4; ++m) am[m] = sfract * wave[0][m];
-            }
-            if (s[1] >= R(0.0)) goto done;
+        for (int m = 0; m < 4; ++m) {
+            R am = k0 * wave[0][m];
+            if (m == mv || m == 3) am = am + k1 * wave[1][m];  // the other components are zero
+            am = am + k1 * wave[2][m];                         // s[2] == s[1]
+            amdq[m] = am + k3 * wave[3][m];
+        }
+        if (!ok) {
+            seldom();
+            ExactIn e;
+            const int at[4] = {0, mu, mv, 3};
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                am[m] = am[m] + s[1] * wave[1][m];
-                am[m] = am[m] + s[2] * wave[2][m];
-            }
-            {
-                const R s3 = cr.vel[mu - 1] + cr.c;  // qR(mu)/rhoi + sqrt(gamma*pi/rhoi)
-                const R rho2 = qR[0] - wave[3][0];
-                const R rhou2 = qR[mu] - wave[3][mu];
-                const R rhov2 = qR[mv] - wave[3][mv];
-                const R en2 = qR[3] - wave[3][3];
-                const R p2 = gamma1 * (en2 - R(0.5) * (rhou2 * rhou2 + rhov2 * rhov2) / rho2);
-                const R c2 = sqrt(gamma * p2 / rho2);
-                const R s2 = rhou2 / rho2 + c2;
-                if (s2 < R(0.0) && s3 > R(0.0)) sfract = s2 * (s3 - s[3]) / (s3 - s2);
-                else if (s[3] < R(0.0)) sfract = s[3];
-                else goto done;
+                e.l[m] = qL[at[m]];
+                e.r[m] = qR[at[m]];
 #pragma unroll
-                for (int m = 0; m < 4; ++m) am[m] = am[m] + sfract * wave[3][m];
+                for (int mw = 0; mw < 4; ++mw) e.w[mw][m] = wave[mw][at[m]];
+                e.s[m] = s[m];
             }
+            const Fluct f = exact_fluct(e, gamma, gamma1);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) amdq[at[m]] = f.am[m];
         }
-    done:
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             R df = s[0] * wave[0][m];
 #pragma unroll
-            for (int mw = 1; mw < W; ++mw) df = df + s[mw] * wave[mw][m];
-            amdq[m] = am[m];
-            apdq[m] = df - am[m];
+            for (int mw = 1; mw < W; ++mw)
+                if (mw != 1 || m == mv || m == 3) df = df + s[mw] * wave[mw][m];  // the shear's other components are zero
+            apdq[m] = df - amdq[m];
         }
+    }
+    // The reference's formulas, components in the order density, normal and
+    // transverse momentum, energy.
+    static __device__ __forceinline__ Roe exact_roe(R l0, R l1, R l2, R l3, R r0, R r1, R r2, R r3, R gamma1) {
+        const R sl = sqrt(l0), sr = sqrt(r0), rhsq2 = sl + sr;
+        const R pl = gamma1 * (l3 - R(0.5) * (l1 * l1 + l2 * l2) / l0);
+        const R pr = gamma1 * (r3 - R(0.5) * (r1 * r1 + r2 * r2) / r0);
+        Roe rr;
+        const R u = rr.u = (l1 / sl + r1 / sr) / rhsq2;
+        const R v = rr.v = (l2 / sl + r2 / sr) / rhsq2;
+        const R enth = rr.enth = ((l3 + pl) / sl + (r3 + pr) / sr) / rhsq2;
+        const R u2v2 = u * u + v * v;
+        const R a2s = gamma1 * (enth - R(0.5) * u2v2);
+        const R a = rr.a = sqrt(a2s);
+        rr.g1a2 = gamma1 / a2s;
+        const R d1 = r0 - l0, d2 = r1 - l1, d3 = r2 - l2, d4 = r3 - l3;
+        rr.a3 = rr.g1a2 * ((enth - u2v2) * d1 + u * d2 + v * d3 - d4);
+        rr.a2 = d3 - v * d1;
+        rr.a4 = (d2 + (a - u) * d1 - a * rr.a3) / (R(2.0) * a);
+        rr.a1 = d1 - rr.a3 - rr.a4;
+        bool in = true;
+        const Dv<R> da(R(2.0) * a, in);
+        rr.y = in ? da.y : R(0.0);
+        return rr;
+    }
+    struct ExactIn { R l[4], r[4], w[4][4], s[4]; };
+    struct Fluct { R am[4]; };
+    static __device__ __forceinline__ Fluct exact_fluct(const ExactIn e, R gamma, R gamma1) {
+        Fluct f;
+        R* am = f.am;
+        const R* s = e.s;
+        const R pl = gamma1 * (e.l[3] - R(0.5) * (e.l[1] * e.l[1] + e.l[2] * e.l[2]) / e.l[0]);
+        const R s0 = e.l[1] / e.l[0] - sqrt(gamma * pl / e.l[0]);
+        R sfract;
+        if (s0 >= R(0.0) && s[0] > R(0.0)) {
+            am[0] = am[1] = am[2] = am[3] = R(0.0);
+            return f;
+        }
+        {
+            const R rho1 = e.l[0] + e.w[0][0];
+            const R rhou1 = e.l[1] + e.w[0][1];
+            const R rhov1 = e.l[2] + e.w[0][2];
+            const R en1 = e.l[3] + e.w[0][3];
+            const R p1 = gamma1 * (en1 - R(0.5) * (rhou1 * rhou1 + rhov1 * rhov1) / rho1);
+            const R c1 = sqrt(gamma * p1 / rho1);
+            const R s1 = rhou1 / rho1 - c1;
+            if (s0 < R(0.0) && s1 > R(0.0)) sfract = s0 * (s1 - s[0]) / (s1 - s0);
+            else if (s[0] < R(0.0)) sfract = s[0];
+            else sfract = R(0.0);
+            for (int m = 0; m < 4; ++m) am[m] = sfract * e.w[0][m];
+        }
+        if (s[1] >= R(0.0)) return f;
+        for (int m = 0; m < 4; ++m) {
+            if (m >= 2) am[m] = am[m] + s[1] * e.w[1][m];  // the other components are zero
+            am[m] = am[m] + s[2] * e.w[2][m];
+        }
+        {
+            const R pr = gamma1 * (e.r[3] - R(0.5) * (e.r[1] * e.r[1] + e.r[2] * e.r[2]) / e.r[0]);
+            const R s3 = e.r[1] / e.r[0] + sqrt(gamma * pr / e.r[0]);
+            const R rho2 = e.r[0] - e.w[3][0];
+            const R rhou2 = e.r[1] - e.w[3][1];
+            const R rhov2 = e.r[2] - e.w[3][2];
+            const R en2 = e.r[3] - e.w[3][3];
+            const R p2 = gamma1 * (en2 - R(0.5) * (rhou2 * rhou2 + rhov2 * rhov2) / rho2);
+            const R c2 = sqrt(gamma * p2 / rho2);
+            const R s2 = rhou2 / rho2 + c2;
+            if (s2 < R(0.0) && s3 > R(0.0)) sfract = s2 * (s3 - s[3]) / (s3 - s2);
+            else if (s[3] < R(0.0)) sfract = s[3];
+            else return f;
+            for (int m = 0; m < 4; ++m) am[m] = am[m] + sfract * e.w[3][m];
+        }
+        return f;
     }
     __device__ __forceinline__ void rpt2(int ixy, const R* asdq, const Roe& rr, R, R,
                                          R* bm, R* bp) const {
         const int mu = (ixy == 1) ? 1 : 2;
         const int mv = (ixy == 1) ? 2 : 1;
         const R u = rr.u, v = rr.v, a = rr.a, enth = rr.enth;
-        const R a3 = rr.g1a2 * (rr.euv * asdq[0] + u * asdq[mu] + v * asdq[mv] - asdq[3]);
+        const R u2v2 = u * u + v * v, euv = enth - u2v2;  // as rpn2 has them
+        const R a3 = rr.g1a2 * (euv * asdq[0] + u * asdq[mu] + v * asdq[mv] - asdq[3]);
         const R a2 = asdq[mu] - u * asdq[0];
-        const R a4 = (asdq[mv] + (a - v) * asdq[0] - a * a3) / (R(2.0) * a);
+        const R x4 = asdq[mv] + (a - v) * asdq[0] - a * a3;
+        bool ok = sizeof(R) == 4 || rr.y != R(0.0);
+        R a4 = Dv<R>(R(2.0) * a, rr.y)(x4, ok);
+        if (!ok) {
+            seldom();
+            a4 = x4 / (R(2.0) * a);
+        }
         const R a1 = asdq[0] - a3 - a4;
         R waveb[4][3], sb[3];
         waveb[0][0] = a1; waveb[mu][0] = a1 * u; waveb[mv][0] = a1 * (v - a); waveb[3][0] = a1 * (enth - v * a);
         sb[0] = v - a;
         waveb[0][1] = a3; waveb[mu][1] = a3 * u + a2; waveb[mv][1] = a3 * v;
-        waveb[3][1] = a3 * R(0.5) * rr.u2v2 + a2 * u; sb[1] = v;
+        waveb[3][1] = a3 * R(0.5) * u2v2 + a2 * u; sb[1] = v;
         waveb[0][2] = a4; waveb[mu][2] = a4 * u; waveb[mv][2] = a4 * (v + a); waveb[3][2] = a4 * (enth + v * a);
         sb[2] = v + a;
 #pragma unroll
@@ -562,7 +797,16 @@ struct GeoclawFwaveT {
     static constexpr bool FWAVE = true;
     static constexpr int M = 3;
     static constexpr int W = 3;
-    struct Roe {};
+    struct Roe { R s[3]; };  // the wave speeds: no Roe averages, there is no transverse solver
+    struct Cell {};
+    static constexpr int NC = 0;
+    static constexpr int NWV = 9;
+    __host__ __device__ static constexpr bool nz(int, int) { return true; }
+    __device__ __forceinline__ void speeds(const Roe& rr, R* s) const {
+        s[0] = rr.s[0];
+        s[1] = rr.s[1];
+        s[2] = rr.s[2];
+    }
     R grav, gamma, gamma1, drytol;
     // one interface of rpn2_geoclaw.f90; the states and bL, bR (aux(1) of the
     // two cells) in FP64
@@ -673,6 +917,41 @@ __device__ __forceinline__ R limiter_phi(int mth, R r) {
             return dmax(R(0.0), dmin(dmin(th * r, (1 + r) / R(2.0)), th));
         }
         default: return dmax(R(0.0), dmin(R(1.0), r));
+    }
+}
+
+// Limiter values of the W waves of an interface: phi(num / wn2) for limiter code
+// lim(mw), 1 where the wave vanishes or is not limited.  The quotients are formed
+// together (fcb_arith.cuh), and again with the operator when one of them leaves
+// the range of that method (a wave of 1e-136 and less).  Where the state is
+// constant, whole warps have no wave and skip all of it.
+template <bool V5, int W, typename R, class LIM>
+__device__ __forceinline__ void limiter_values(const R* num, const R* wn2, const LIM& lim, R* phi) {
+    bool any = false;
+#pragma unroll
+    for (int mw = 0; mw < W; ++mw) {
+        phi[mw] = R(1);
+        any = any | (wn2[mw] != R(0));
+    }
+    if (any) {
+        bool ok = true;
+        R r[W];
+#pragma unroll
+        for (int mw = 0; mw < W; ++mw) {
+            const Dv<R> d(wn2[mw] == R(0) ? R(1) : wn2[mw], ok);
+            r[mw] = d(num[mw], ok);
+        }
+        if (!ok) {
+            seldom();
+#pragma unroll
+            for (int mw = 0; mw < W; ++mw) r[mw] = num[mw] / wn2[mw];
+        }
+#pragma unroll
+        for (int mw = 0; mw < W; ++mw) {
+            const int mth = lim(mw);
+            const R p = limiter_phi((V5 && mth > 5) ? 1 : mth, r[mw]);
+            phi[mw] = (mth == 0 || wn2[mw] == R(0)) ? R(1) : p;
+        }
     }
 }
 

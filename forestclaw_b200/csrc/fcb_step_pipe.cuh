@@ -57,13 +57,13 @@ struct Method {
     __device__ __forceinline__ int lim(int mw) const { return LIM > 0 ? LIM : a.mthlim[mw]; }
 };
 
-// psi at a node: (sin^2(pi x) sin^2(pi y))/pi.  The FP64 form divides as the
-// reference does; the mixed form multiplies by 1/pi (one more rounding, far
-// below its FP32 solves).
+// psi at a node: (sin^2(pi x) sin^2(pi y))/pi.  The FP64 form rounds the quotient as
+// the reference's division does (div_pi); the mixed form multiplies by 1/pi (one
+// more rounding, far below its FP32 solves).
 template <typename R>
 __device__ __forceinline__ double psi_node(double tx, double ty) {
     constexpr double pi = 3.141592653589793;  // 4*atan(1) in double precision
-    if constexpr (sizeof(R) == sizeof(double)) return (tx * ty) / pi;
+    if constexpr (sizeof(R) == sizeof(double)) return div_pi(tx * ty);
     else return (tx * ty) * (1.0 / pi);
 }
 
@@ -391,26 +391,26 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 for (int m = 0; m < M; ++m) cq[m] = R(0);
                 if (meth.second_order()) {
                     if (c >= MBC && c <= MBC + MX) {
+                        R num[W], wn2[W], phi[W];
 #pragma unroll
                         for (int mw = 0; mw < W; ++mw) {
-                            const int mth = meth.lim(mw);
-                            if (mth == 0) continue;
-                            R wn2 = S.xwl[mw][0] * S.xwl[mw][0];
+                            wn2[mw] = S.xwl[mw][0] * S.xwl[mw][0];
                             R dl = xw[(mw * M + 0) * L::PNX - 1] * S.xwl[mw][0];
                             R dr = S.xwl[mw][0] * xw[(mw * M + 0) * L::PNX + 1];
 #pragma unroll
                             for (int m = 1; m < M; ++m) {
                                 const R wc = S.xwl[mw][m];
-                                wn2 = wn2 + wc * wc;
+                                wn2[mw] = wn2[mw] + wc * wc;
                                 dl = dl + xw[(mw * M + m) * L::PNX - 1] * wc;
                                 dr = dr + wc * xw[(mw * M + m) * L::PNX + 1];
                             }
-                            if (wn2 == R(0)) continue;
-                            const R rr = (S.xsl[mw] > R(0)) ? dl / wn2 : dr / wn2;
-                            const R phi = limiter_phi((SOL::V5 && mth > 5) ? 1 : mth, rr);
-#pragma unroll
-                            for (int m = 0; m < M; ++m) S.xwl[mw][m] = phi * S.xwl[mw][m];
+                            num[mw] = (S.xsl[mw] > R(0)) ? dl : dr;
                         }
+                        limiter_values<SOL::V5, W>(num, wn2, [&](int mw) { return meth.lim(mw); }, phi);
+#pragma unroll
+                        for (int mw = 0; mw < W; ++mw)
+#pragma unroll
+                            for (int m = 0; m < M; ++m) S.xwl[mw][m] = phi[mw] * S.xwl[mw][m];
                     }
 #pragma unroll
                     for (int m = 0; m < M; ++m) {
@@ -580,19 +580,19 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
             for (int m = 0; m < M; ++m) cq[m] = R(0);
             if (meth.second_order() && fact) {
                 if (inner) {
+                    R num[W], wn2[W], phi[W];
 #pragma unroll
                     for (int mw = 0; mw < W; ++mw) {
-                        const int mth = meth.lim(mw);
-                        if (mth == 0) continue;
-                        R wn2 = S.yw_f[mw][0] * S.yw_f[mw][0];
+                        wn2[mw] = S.yw_f[mw][0] * S.yw_f[mw][0];
 #pragma unroll
-                        for (int m = 1; m < M; ++m) wn2 = wn2 + S.yw_f[mw][m] * S.yw_f[mw][m];
-                        if (wn2 == R(0)) continue;
-                        const R rr = (S.ys_f[mw] > R(0)) ? S.ydotl[mw] / wn2 : ydotr[mw] / wn2;
-                        const R phi = limiter_phi((SOL::V5 && mth > 5) ? 1 : mth, rr);
-#pragma unroll
-                        for (int m = 0; m < M; ++m) w[mw][m] = phi * w[mw][m];
+                        for (int m = 1; m < M; ++m) wn2[mw] = wn2[mw] + S.yw_f[mw][m] * S.yw_f[mw][m];
+                        num[mw] = (S.ys_f[mw] > R(0)) ? S.ydotl[mw] : ydotr[mw];
                     }
+                    limiter_values<SOL::V5, W>(num, wn2, [&](int mw) { return meth.lim(mw); }, phi);
+#pragma unroll
+                    for (int mw = 0; mw < W; ++mw)
+#pragma unroll
+                        for (int m = 0; m < M; ++m) w[mw][m] = phi[mw] * w[mw][m];
                 }
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
