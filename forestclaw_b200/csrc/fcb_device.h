@@ -46,6 +46,16 @@ struct FuseNbr {
     int32_t bc[4];
 };
 
+// Ghost-exchange fusion on a mesh of one level: the mesh as one grid of n x n
+// cells (2^lgp patches of 2^lg cells a side), swept in nsx x nsy strips of w x h.
+struct StripArgs {
+    const int32_t* grid;  // slot of patch (x, y) at y * 2^lgp + x; null: not a fused step
+    int32_t n, lg, lgp, nxp;  // nxp: columns of a patch with its ghost columns
+    int32_t bc[4];        // mthbc of the domain's sides (left, right, bottom, top), 0: periodic
+    double ax, ay;        // lower-left corner of the domain
+    int32_t w, h, nsx, nsy;  // set by the launcher
+};
+
 // Arguments of one batched step launch (all patches of one level).
 struct StepArgs {
     double* q;             // arena base
@@ -78,6 +88,7 @@ struct StepArgs {
     // the arena q (qsrc != q)
     const double* qsrc;
     const FuseNbr* fuse;
+    StripArgs strip;
     // four-barrier form: nbands > 1 splits every patch's rows into that many
     // bands, one CTA each, which read the copy qsrc of the arena (bands
     // overlap in the rows they read) and update their own rows in q
@@ -90,6 +101,7 @@ struct StepArgs {
     // the launcher split the last, partial wave of CTAs into row bands (the
     // patches of that tail are copied there and read from it); null: off
     double* qtail;
+    int32_t ppc;           // split form: patches per CTA of this launch
 };
 
 // Conservation registers of one slot (fclaw2d_clawpatch_registers_t), doubles

@@ -1440,9 +1440,10 @@ void Context::launch_step_form(const StepArgs& a, int n) {
         if (aux_kind_ == AUX_SWIRL) e = launch_step_warp_swirl(opt_.mx, opt_.mbc, a, st_);
         if (e == cudaErrorNotSupported) throw Error(FCB_ERR_INVALID, "no warp-synchronous step for this case");
     } else if (v == 3) {
-        // default: the pipelined form for scalar advection; the Roe solvers keep
-        // the four-barrier form, whose smaller register footprint suits them
-        e = launch_step_pipe(opt_.solver_kind, aux_kind_, opt_.mwaves, opt_.mx, opt_.my, opt_.mbc, opt_.claw_version,
+        // patches of mx = 64 have a pipelined form for the Roe systems alone, which
+        // the library chooses itself (step_variant 3 has always refused them)
+        if (opt_.step_variant == 0 || opt_.mx <= 32)
+            e = launch_step_pipe(opt_.solver_kind, aux_kind_, opt_.mwaves, opt_.mx, opt_.my, opt_.mbc, opt_.claw_version,
                              a, st_);
         if (e == cudaErrorNotSupported && v == 3) throw Error(FCB_ERR_INVALID, "no pipelined step for this case");
     }
@@ -1764,10 +1765,7 @@ std::map<std::vector<int>, int> g_step_form_cache, g_ghost_unroll_cache;
 
 int default_step_form(const fcb_options_t& o) {
     if (o.solver_kind == SOLVER_ADVECTION_MANIFOLD) return 1;  // capacity: four-barrier form only
-    return (o.solver_kind == SOLVER_ADVECTION || o.claw_version == 5 || o.solver_kind == SOLVER_GEOCLAW_FWAVE ||
-            o.precision == 1)
-               ? 3
-               : 1;
+    return 3;
 }
 }  // namespace
 
@@ -1787,20 +1785,14 @@ int Context::tune_step_form(const StepArgs& a, int n) {
     // +1 % (shallow water) and -12 % (Euler) on the AMR configurations, whose
     // level updates are bound by the SMs' throughput at one 255-register CTA
     // each, not by the length of one CTA's row sweep.
-    // The Roe systems of clawpack 4.6 in FP64 run the four-barrier form: since
-    // it shares the per-cell quantities of the Riemann problems it measured
-    // faster than the pipelined form at every size on B200 (shallow water
-    // mx = 32 about 2x, Euler 1.01-1.9x), and a choice between the two made
-    // per octave of the patch count could flip on a close race at one size and
-    // cost 2x at another (a one-wave four-barrier launch against a two-wave
-    // pipelined one), so the pipelined form is not tried for them.
+    // The systems run the pipelined form with both sweeps of a column on two threads
+    // (fcb_step_split.cuh), faster than the four-barrier form at every size measured on
+    // B200: shallow water mx = 32, 1,024 patches 0.139 against 0.395 ms, 4 patches 0.080
+    // against 0.185 ms; Euler mx = 16, 4,096 patches 0.320 against 0.856 ms.
     std::vector<int> cand;
     if (opt_.solver_kind == SOLVER_ADVECTION_MANIFOLD) cand = {1};  // capacity: four-barrier form only
-    else if (opt_.precision == 1 || opt_.claw_version == 5 || opt_.solver_kind == SOLVER_GEOCLAW_FWAVE) cand = {3};
+    else if (opt_.precision == 1 || opt_.claw_version == 5 || opt_.solver_kind != SOLVER_ADVECTION) cand = {3};
     else if (aux_kind_ == AUX_SWIRL) cand = {1, 2, 3};
-    else if (opt_.solver_kind == SOLVER_SWE_ROE || opt_.solver_kind == SOLVER_EULER4_ROE ||
-             opt_.solver_kind == SOLVER_ADVECTION_MANIFOLD)
-        cand = {1};
     else cand = {1, 3};
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(st_, &cs);
@@ -2310,14 +2302,9 @@ cudaError_t launch_step_batch(const fcb_options_t& opt, int aux_kind, const Patc
     a.gamma1 = opt.gamma - 1.0;
     a.drytol = opt.dry_tolerance;
     a.cfl_out = d_cfl;
-    // the Roe systems of clawpack 4.6 in FP64 run the four-barrier CTA form (on
-    // B200 about twice the pipelined form's rate for shallow water at mx = 32)
-    // (capacity exists in that form only, clawpack 4.6 and 5)
+    // capacity exists in the four-barrier form only, clawpack 4.6 and 5
     if (opt.solver_kind == FCB_SOLVER_ADVECTION_MANIFOLD)
         return launch_step(opt.solver_kind, aux_kind, opt.mwaves, opt.mx, opt.my, opt.mbc, a, st, opt.claw_version);
-    if (opt.precision != 1 && opt.claw_version != 5 &&
-        (opt.solver_kind == FCB_SOLVER_SWE_ROE || opt.solver_kind == FCB_SOLVER_EULER4_ROE))
-        return launch_step(opt.solver_kind, aux_kind, opt.mwaves, opt.mx, opt.my, opt.mbc, a, st);
     return opt.precision == 1
                ? launch_step_pipe_mixed(opt.solver_kind, aux_kind, opt.mwaves, opt.mx, opt.my, opt.mbc,
                                         opt.claw_version, a, st)

@@ -40,6 +40,12 @@
 
 namespace fcb {
 
+// the systems' pipelined form (fcb_step_split.cuh)
+cudaError_t launch_split_swe(int mx, int claw_version, const StepArgs& a, cudaStream_t st);
+cudaError_t launch_split_geoclaw(int mx, const StepArgs& a, cudaStream_t st);
+cudaError_t launch_split_euler(int mx, int claw_version, const StepArgs& a, cudaStream_t st);
+cudaError_t launch_split_mixed(int solver, int mx, int claw_version, const StepArgs& a, cudaStream_t st);
+
 namespace {
 
 __device__ __forceinline__ void atomic_max_nonneg_p(unsigned long long* p, double v) {
@@ -1003,18 +1009,24 @@ cudaError_t launch_step_pipe_v(int solver, int aux_kind, int mwaves, int mx, int
             return cudaErrorNotSupported;
         case SOLVER_SWE_ROE:
             if (mwaves != 3 || aux_kind != AUX_NONE) return cudaErrorNotSupported;
-            return launch_pipe_mx<SweRoeT<R, V5>, AUX_NONE, 0, FUSED>(mx, mbc, a, st);
+            if constexpr (FUSED) return launch_pipe_mx<SweRoeT<R, V5>, AUX_NONE, 0, FUSED>(mx, mbc, a, st);
+            break;
         case SOLVER_EULER4_ROE:
             if (mwaves != 4 || aux_kind != AUX_NONE) return cudaErrorNotSupported;
-            return launch_pipe_mx<Euler4RoeT<R, V5>, AUX_NONE, 0, FUSED>(mx, mbc, a, st);
+            if constexpr (FUSED) return launch_pipe_mx<Euler4RoeT<R, V5>, AUX_NONE, 0, FUSED>(mx, mbc, a, st);
+            break;
         case SOLVER_GEOCLAW_FWAVE:
-            if constexpr (!V5) {
-                if (mwaves != 3 || aux_kind != AUX_STORED || a.maux != 1) return cudaErrorNotSupported;
-                return launch_pipe_mx<GeoclawFwaveT<R>, AUX_STORED, 1, FUSED>(mx, mbc, a, st);
-            }
-            return cudaErrorNotSupported;
+            if (V5 || mwaves != 3 || aux_kind != AUX_STORED || a.maux != 1) return cudaErrorNotSupported;
+            if constexpr (FUSED && !V5) return launch_pipe_mx<GeoclawFwaveT<R>, AUX_STORED, 1, FUSED>(mx, mbc, a, st);
+            break;
         default: return cudaErrorNotSupported;
     }
+    // the unfused systems: both sweeps of a column on two threads
+    if (mbc != 2) return cudaErrorNotSupported;
+    if constexpr (std::is_same_v<R, float>) return launch_split_mixed(solver, mx, V5 ? 5 : 4, a, st);
+    else if (solver == SOLVER_SWE_ROE) return launch_split_swe(mx, V5 ? 5 : 4, a, st);
+    else if (solver == SOLVER_EULER4_ROE) return launch_split_euler(mx, V5 ? 5 : 4, a, st);
+    else return launch_split_geoclaw(mx, a, st);
 }
 
 // FUSED: the ghost-exchange-fused form (a.fuse and a.qsrc set; mesh of one level)
