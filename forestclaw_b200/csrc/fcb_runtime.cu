@@ -486,7 +486,7 @@ void Context::mesh_changed() {
     h_groups_.clear();
     h_xitems_.clear();
     ops_dirty_ = true;
-    build_fuse_table();
+    build_strip_grid();
 }
 
 // ---------------------------------------------------------------------------
@@ -1950,55 +1950,67 @@ int Context::tune_ghost_unroll(const GhostPlan& g) {
 // On such a mesh every macro step is n_fine level updates, each followed by a
 // ghost update whose records are same-size copies and physical boundary
 // conditions only (fclaw2d_advance.c:285-341 with one level).  The fused step
-// reads each patch's ghost cells from its neighbours' interiors through a
-// per-slot table (the values those records would write), reads from one arena
-// and writes the updated interiors into the other, so no patch reads a
-// neighbour that the same launch has already updated.  The ghost cells the
+// sweeps the mesh in strips that cross patch edges (fcb_step_pipe.cuh), finding
+// patches through a table of the mesh; it reads interior cells of one arena (the
+// values those records would copy) and writes them in the other, so no strip
+// reads a cell that the same launch has already updated.  The ghost cells the
 // reference's step would also update are dead: the following ghost update
 // overwrites every one of them.  The last ghost update of the macro step is
 // recorded and run by ensure_ghosts() before anything reads ghost cells, so
 // every array a caller sees equals the unfused result bit for bit.
 // ---------------------------------------------------------------------------
-void Context::build_fuse_table() {
-    fuse_ok_ = false;
-    if (partitioned() || gmin_ != gmax_ || own_count_ <= 0 || capacity_ <= 0) return;
-    std::vector<FuseNbr> t((size_t)capacity_);
-    for (auto& f : t) {
-        for (int k = 0; k < 4; ++k) f.face[k] = f.corner[k] = -1;
-        for (int k = 0; k < 4; ++k) f.bc[k] = 0;
-    }
+void Context::build_strip_grid() {
+    strip_ = StripArgs{};
+    if (partitioned() || gmin_ != gmax_ || own_count_ <= 0 || num_patches() != (1 << (2 * gmax_))) return;
+    const int P = 1 << gmax_;
+    strip_.lgp = gmax_;
+    while ((1 << strip_.lg) < opt_.mx) ++strip_.lg;
+    strip_.n = opt_.mx << gmax_;
+    strip_.nxp = nx_;
+    strip_.ax = opt_.ax;
+    strip_.ay = opt_.ay;
+    for (int k = 0; k < 4; ++k) strip_.bc[k] = (k < 2 ? opt_.periodic_x : opt_.periodic_y) ? 0 : opt_.mthbc[k];
+    // a strip takes every cell size and position from the domain's corner and one
+    // spacing: the patches' own must be the same numbers, which they are when the
+    // cell edges and centres are exact in double precision
+    const double dx = h_meta_[slot_of_[0]].dx, dy = h_meta_[slot_of_[0]].dy;
+    auto exact = [&](double lo, double hi, double d) {
+        int e;
+        std::frexp(d, &e);
+        const double ulp = std::ldexp(1.0, e - 53);  // d is a multiple of it
+        double unit = ulp;
+        while (std::fmod(d, 2.0 * unit) == 0.0) unit *= 2.0;
+        unit *= 0.5;  // half cells: the centres
+        return std::fmod(lo, unit) == 0.0 &&
+               std::max(std::fabs(lo), std::fabs(hi)) + 4.0 * d <= std::ldexp(unit, 53);
+    };
+    if (!exact(opt_.ax, opt_.bx, dx) || !exact(opt_.ay, opt_.by, dy)) return;
+    std::vector<int32_t> grid((size_t)P * P, -1);
+    const int sh = QuadForest::kMaxLevel - gmax_;
     for (int p = 0; p < num_patches(); ++p) {
-        const Neighbors& nb = nbrs_[p];
-        FuseNbr f;
-        for (int k = 0; k < 4; ++k) {
-            f.bc[k] = 0;
-            f.face[k] = f.corner[k] = -1;
-            if (nb.face_rel[k] == REL_BOUNDARY) f.bc[k] = opt_.mthbc[k];
-            else if (nb.face_rel[k] == REL_SAMESIZE) f.face[k] = slot_of_[nb.face_nbr[k][0]];
-            else return;  // a coarse/fine face: not a mesh of one level
-            if (nb.corner_rel[k] == REL_SAMESIZE) f.corner[k] = slot_of_[nb.corner_nbr[k]];
-        }
-        // a corner block is copied from the corner neighbour unless one of its
-        // two faces is a physical boundary; that neighbour must exist
-        for (int c = 0; c < 4; ++c) {
-            const int fx = (c & 1) ? 1 : 0, fy = (c & 2) ? 3 : 2;
-            if (f.bc[fx] == 0 && f.bc[fy] == 0 && f.corner[c] < 0) return;
-        }
-        t[slot_of_[p]] = f;
+        const Leaf& l = forest_.leaves[p];
+        const PatchMeta& m = h_meta_[slot_of_[p]];
+        const int px = l.x >> sh, py = l.y >> sh;
+        if (m.dx != dx || m.dy != dy || m.xlower != opt_.ax + (double)(px * opt_.mx) * dx ||
+            m.ylower != opt_.ay + (double)(py * opt_.my) * dy)
+            return;
+        grid[(size_t)py * P + px] = slot_of_[p];
     }
-    d_fuse_.reserve((size_t)capacity_);
-    check(cudaMemcpy(d_fuse_.p, t.data(), t.size() * sizeof(FuseNbr), cudaMemcpyHostToDevice), "fuse table");
-    fuse_ok_ = true;
+    d_grid_.reserve(grid.size());
+    check(cudaMemcpy(d_grid_.p, grid.data(), grid.size() * sizeof(int32_t), cudaMemcpyHostToDevice), "strip grid");
+    strip_.grid = d_grid_.p;
 }
 
 bool Context::fusion_possible() const {
     // the fused step reads the neighbours' interiors where the unfused one
     // reads its own ghost cells: equal only when those hold a ghost update's values
-    return opt_.ghost_fusion != 1 && fuse_ok_ && ghosts_filled_ && !partitioned() && !time_sync_ && !dry_ &&
+    return opt_.ghost_fusion != 1 && strip_.grid && ghosts_filled_ && !partitioned() && !time_sync_ && !dry_ &&
            opt_.src_term == 0 &&
            gmin_ == gmax_ &&
            own_count_ > 0 && (opt_.step_variant == 0 || opt_.step_variant == 3) && opt_.mbc == 2 &&
-           (opt_.mx == 8 || opt_.mx == 16 || opt_.mx == 32);
+           // mx = 64 exists for clawpack 4.6 in FP64, in the library's own choice of form
+           (opt_.mx <= 32 || (opt_.step_variant == 0 && opt_.precision == 0 && opt_.claw_version == 4 &&
+                              opt_.solver_kind != FCB_SOLVER_GEOCLAW_FWAVE));
 }
 
 namespace {
@@ -2040,7 +2052,7 @@ void Context::launch_fused_step(double t, double dt, const double* src, double* 
     fill_step_args(a, t, dt, cfl_slot);
     a.q = dst;
     a.qsrc = src;
-    a.fuse = d_fuse_.p;
+    a.strip = strip_;
     a.slots = d_level_slots_.p + b;
     a.npatches = e - b;
     cudaError_t r = opt_.precision == 1

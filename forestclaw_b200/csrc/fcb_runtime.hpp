@@ -38,7 +38,7 @@ cudaError_t launch_step_pipe(int solver, int aux_kind, int mwaves, int mx, int m
                              const StepArgs& a, cudaStream_t st);
 cudaError_t launch_step_pipe_mixed(int solver, int aux_kind, int mwaves, int mx, int my, int mbc,
                                    int claw_version, const StepArgs& a, cudaStream_t st);
-// the ghost-exchange-fused pipelined forms (a.fuse, a.qsrc set; a mesh of one level)
+// the ghost-exchange-fused pipelined forms (a.strip, a.qsrc set; a mesh of one level)
 cudaError_t launch_step_pipe_fused(int solver, int aux_kind, int mwaves, int mx, int my, int mbc, int claw_version,
                                    const StepArgs& a, cudaStream_t st);
 cudaError_t launch_step_pipe_fused_mixed(int solver, int aux_kind, int mwaves, int mx, int my, int mbc,
@@ -291,8 +291,8 @@ class Context {
     DevBuf<double> d_xsend_, d_xrecv_;
     double launch_level_step(int level, double t, double dt, unsigned long long* cfl_slot);
     // --- ghost-exchange fusion on a mesh of one level ---
-    // The fused step reads arena d_q_ (ghost cells through the neighbour table
-    // d_fuse_) and writes the interiors into d_qalt_; the two are then swapped.
+    // The fused step reads the interiors of arena d_q_ (patches found through the
+    // mesh's table d_grid_) and writes those of d_qalt_; the two are then swapped.
     // The ghost update that would follow is recorded (ghosts_stale_) and run by
     // ensure_ghosts() before anything reads ghost cells.
     bool fusion_possible() const;             // mesh, options and step form allow it
@@ -303,15 +303,15 @@ class Context {
     // device time of `launches` step launches (fused: the fused step; with_fill:
     // the unfused step followed by the ghost fill) on scratch copies of q
     double time_steps(bool fused, bool with_fill, int launches, double t, double dt);
-    void build_fuse_table();
+    void build_strip_grid();
     void fill_step_args(StepArgs& a, double t, double dt, unsigned long long* cfl_slot) const;
     void launch_step_form(const StepArgs& a, int n);
   public:
     void ensure_ghosts();  // run the deferred ghost update, if one is pending
   private:
     double* d_qalt_ = nullptr;
-    DevBuf<FuseNbr> d_fuse_;
-    bool fuse_ok_ = false;        // the table of the current mesh is complete
+    DevBuf<int32_t> d_grid_;      // slots of a mesh of one level by place
+    StripArgs strip_{};           // grid null: the mesh has no strips
     bool ghosts_stale_ = false;
     int stale_min_ = 0, stale_max_ = 0;
     double stale_t_ = 0.0;

@@ -33,10 +33,13 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "fcb_device.h"
 #include "fcb_solvers.cuh"
+#include "fcb_strip.cuh"
 
 namespace fcb {
 
@@ -97,9 +100,9 @@ struct PipeSmem {
     static constexpr int DBYTES = ((NR * (int)sizeof(R) + 15) / 16) * 16;
     static constexpr int GY = 0;                      // 4 slots x 2M: y transverse sums
     static constexpr int NDS = PPB * (NX + 1);
-    static constexpr int TY = GY + 4 * 2 * M * PNX;   // swirl: sin^2 of the node rows [patch][NX+1]
-    static constexpr int ND = TY + (SWIRL ? NDS : 0); // swirl: psi node rows, 2 slots [patch][NX+1]
-    static constexpr int NDEND = ND + (SWIRL ? 2 * NDS : 0);
+    static constexpr int ND = GY + 4 * 2 * M * PNX;         // swirl: psi node rows, 2 slots [patch][NX+1]
+    static constexpr int TY = ND + (SWIRL ? 2 * NDS : 0);   // swirl: sin^2 of the node rows [patch][NX+1]; last,
+    static constexpr int NDEND = TY + (SWIRL ? NDS : 0);    // since a strip's has its rows + 1 entries instead
     static constexpr int Q = QDBL ? NDEND : 0;
     static constexpr int AX = QDBL ? NDEND + 2 * M * PNX : AXR;
     static constexpr int BYTES = DBYTES + (QDBL ? NDEND + 2 * M * PNX + 4 * NAUX * PNX : NDEND) * 8;
@@ -130,16 +133,17 @@ struct PipeState {
     double pcur;                                         // swirl: psi at node (c, s+1)
     R smax_x, smax_y;  // largest |s| over the CFL interfaces of each direction
     bool bad;          // a Riemann problem the reference would stop on (reported as a NaN CFL)
+    int sslot, dslot;  // strip form: slots of the patches this column reads and writes now
 };
 
 // Per-thread constants: column, flags and this thread's element of the rings.
 template <typename R>
 struct PipeThread {
-    double* q;        // q of the patch, offset to column c (fused: the patch in the arena written)
+    double* q;        // q of the patch, offset to column c (strip form: the arena written)
     double* qlast;    // qlast of the patch, offset to column c
-    const double* qs; // fused: where rows MBC..MBC+MX-1 of column c are read (neighbour or own patch)
-    unsigned negmid;  // fused: components negated on those rows (bit m: component m; solid walls)
-    int slot;         // fused: the patch's slot
+    int x, xm, y0;    // strip form: mesh column the values come from, the column itself, first interior row
+    unsigned negx;    // strip form: components negated in this column (solid walls)
+    int mx, ny;       // interior columns and rows (ghost rows included) of the patch or strip
     const double* aux;
     R* rb;            // this thread's element of the R rings
     double* db;       // this thread's element of the FP64 rings
@@ -164,97 +168,47 @@ __host__ __device__ constexpr bool pipe_time_sync() {
 // ring slot of row s - d when s == J (mod D) is known at compile time
 __host__ __device__ constexpr int cslot(int J, int d, int D) { return ((J - d) % D + D) % D; }
 
-// Ghost-exchange fusion: where cell (c, s) of the patch in `slot` gets its
-// value when the ghost update that precedes the step is folded into the step.
-// On a mesh of one level that update (fclaw2d_ghost_update_async, one rank)
-// first copies the same-size neighbours' interior cells into the face bands
-// and corner blocks (fclaw2d_clawpatch46_fort_copy_face/_corner, the
-// same-block transform a shift by mx), then applies the physical boundary
-// conditions (clawpack46_bc2_default.f) left, right, bottom, top, each over the
-// whole band including the corner cells.  The bottom/top conditions are
-// applied last, so they are resolved first: a cell of a physical bottom band
-// takes row 1 (extrapolation) or the mirrored row (wall, component 3 negated);
-// then a physical left/right band takes column 1 / mx or the mirrored column
-// (wall, component 2 negated); whatever still lies outside the interior is
-// the copy from the face or corner neighbour that owns it.  *p receives the
-// address of component 0 of the source cell in the arena qsrc; bit m of *neg
-// says that component m is negated.
-template <int MX, int MBC>
-__device__ __forceinline__ void fused_src(const StepArgs& a, int slot, int c, int s, const double*& p,
-                                          unsigned& neg) {
-    constexpr int NX = MX + 2 * MBC;
-    constexpr int HI = MBC + MX;  // first ghost row / column after the interior
-    const FuseNbr* F = a.fuse + slot;
-    int col = c, row = s, sl = slot;
-    neg = 0u;
-    if (row < MBC) {
-        const int bc = __ldg(&F->bc[2]);
-        if (bc == 3) { row = 2 * MBC - 1 - row; neg ^= 4u; }
-        else if (bc != 0) row = MBC;
-    } else if (row >= HI) {
-        const int bc = __ldg(&F->bc[3]);
-        if (bc == 3) { row = 2 * HI - 1 - row; neg ^= 4u; }
-        else if (bc != 0) row = HI - 1;
-    }
-    if (col < MBC) {
-        const int bc = __ldg(&F->bc[0]);
-        if (bc == 3) { col = 2 * MBC - 1 - col; neg ^= 2u; }
-        else if (bc != 0) col = MBC;
-    } else if (col >= HI) {
-        const int bc = __ldg(&F->bc[1]);
-        if (bc == 3) { col = 2 * HI - 1 - col; neg ^= 2u; }
-        else if (bc != 0) col = HI - 1;
-    }
-    const int h = col < MBC ? 0 : (col >= HI ? 2 : 1);
-    const int v = row < MBC ? 0 : (row >= HI ? 2 : 1);
-    if (h != 1 || v != 1) {
-        int n;
-        if (v == 1) n = __ldg(&F->face[h == 0 ? 0 : 1]);
-        else if (h == 1) n = __ldg(&F->face[v == 0 ? 2 : 3]);
-        else n = __ldg(&F->corner[(v == 0 ? 0 : 2) + (h == 0 ? 0 : 1)]);
-        if (n >= 0) {  // always on a complete table; otherwise the patch's own (stale) ghost cell
-            sl = n;
-            col += h == 0 ? MX : (h == 2 ? -MX : 0);
-            row += v == 0 ? MX : (v == 2 ? -MX : 0);
-        }
-    }
-    p = a.qsrc + (int64_t)sl * a.q_stride + (int64_t)row * NX + col;
-}
-
-// Component m of row `row` of this thread's column as the step sees it.
-template <int MX, int MBC, bool FUSED, typename R>
-__device__ __forceinline__ double load_q(const StepArgs& a, const PipeThread<R>& T, int m, int row) {
-    constexpr int NX = MX + 2 * MBC;
-    constexpr int NY = NX;
+// Row `row` of this thread's column (every component).  Strip form: rows come in
+// order, and the slot is looked up again at patch edges and outside the domain.
+template <class SOL, int NX, bool FUSED>
+__device__ __forceinline__ void load_row(const StepArgs& a, const PipeThread<typename SOL::Real>& T, PipeState<SOL>& S,
+                                         int row, double* v) {
+    constexpr int M = SOL::M;
     if constexpr (!FUSED) {
-        return T.q[((int64_t)m * NY + row) * NX];
+#pragma unroll
+        for (int m = 0; m < M; ++m) v[m] = T.q[((int64_t)m * NX + row) * NX];
     } else {
-        if (row >= MBC && row < MBC + MX) {
-            const double v = T.qs[((int64_t)m * NY + row) * NX];
-            return ((T.negmid >> m) & 1u) ? -v : v;
+        const StripArgs& g = a.strip;
+        const int ym = T.y0 - 2 + row;
+        bool wall;
+        const int y = strip_inside(ym, g.n, g.bc[2], g.bc[3], wall);
+        if (row == 0 || ym <= 0 || ym >= g.n || (y & ((1 << g.lg) - 1)) == 0) S.sslot = strip_slot(g, T.x, y);
+        const double* p = a.qsrc + ((int64_t)S.sslot * a.q_stride + strip_cell(g, T.x, y));
+        const int plane = g.nxp * g.nxp;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            v[m] = p[m * plane];
+            if constexpr (M > 1)
+                if (((T.negx ^ (wall ? 4u : 0u)) >> m) & 1u) v[m] = -v[m];
         }
-        const double* p;
-        unsigned neg;
-        fused_src<MX, MBC>(a, T.slot, T.c, row, p, neg);
-        const double v = p[(int64_t)m * NY * NX];
-        return ((neg >> m) & 1u) ? -v : v;
     }
 }
 
 // One row-iteration.  J >= 0: s == J (mod 4) at compile time, so every ring
 // slot is a constant; STEADY: s in [4, NY-2], where every stage is active for
 // every row and the row-range tests vanish.
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int PPB, int LIM, int J, bool STEADY, bool FUSED>
+template <class SOL, int NX, int MBC, int AUXK, int NAUX, int PPB, int LIM, int J, bool STEADY, bool FUSED>
 __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                                           const PipeThread<typename SOL::Real>& T, PipeState<SOL>& S, int s) {
     using R = typename SOL::Real;
     using QT = ring_t<SOL>;
     constexpr int M = SOL::M;
     constexpr int W = SOL::W;
-    constexpr int NX = MX + 2 * MBC;
-    constexpr int NY = NX;
     constexpr bool SWIRL = AUXK == AUX_SWIRL;
     constexpr bool QDBL = ring_in_fp64<SOL>;
+    // a patch's size is known at compile time, a strip's is not
+    const int MX = FUSED ? T.mx : NX - 2 * MBC, MY = FUSED ? T.ny - 2 * MBC : NX - 2 * MBC;
+    const int NXL = MX + 2 * MBC, NY = MY + 2 * MBC;
     using L = PipeSmem<NX, PPB, M, W, NAUX, SWIRL, R, QDBL>;
     QT* qb;  // this thread's element of the state and aux rings
     if constexpr (QDBL) qb = T.db;
@@ -286,18 +240,29 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
     // a fused step writes the interior cells only: the ghost cells it would
     // update are overwritten by the ghost update that follows every step on a
     // mesh of one level, and that update is deferred until the ghost cells are read
-    const bool upd = T.active && ((V5 || FUSED) ? (s - 4 >= MBC && s - 4 <= MBC + MX - 1 && c >= MBC && c <= MBC + MX - 1)
+    const bool upd = T.active && ((V5 || FUSED) ? (s - 4 >= MBC && s - 4 <= MBC + MY - 1 && c >= MBC && c <= MBC + MX - 1)
                                                 : ((STEADY || (s - 4 >= 0 && s - 4 <= NY - 2)) && c <= NX - 2));
+    int64_t dst = 0;  // strip form: where cell (c, s-4) lives in the arenas
+    if constexpr (FUSED) {
+        if (upd) {
+            const int y = T.y0 + s - 4 - MBC;
+            if (s - 4 == MBC || (y & ((1 << a.strip.lg) - 1)) == 0) S.dslot = strip_slot(a.strip, T.x, y);
+            dst = (int64_t)S.dslot * a.q_stride + strip_cell(a.strip, T.x, y);
+        }
+    }
     {
-        // prefetch two rows ahead; the last steady iteration (s = 4 + 4*((NY-5)/4) - 1)
-        // still has row s+2 inside the patch for the patch sizes built here
-        constexpr bool STEADY_IN = 4 + 4 * ((NY - 5) / 4) + 1 < NY;
+        // prefetch two rows ahead; the last steady iteration of a patch
+        // (s = 4 + 4*((NY-5)/4) - 1) still has row s+2 inside it for the sizes built here
+        constexpr bool STEADY_IN = !FUSED && 4 + 4 * ((NX - 5) / 4) + 1 < NX;
         const bool on = T.active && ((STEADY && STEADY_IN) || s + 2 < NY);
 #pragma unroll
+        for (int m = 0; m < M; ++m) qnext[m] = 0.0;
+        if (on) load_row<SOL, NX, FUSED>(a, T, S, s + 2, qnext);
+#pragma unroll
         for (int m = 0; m < M; ++m) {
-            qnext[m] = on ? load_q<MX, MBC, FUSED>(a, T, m, s + 2) : 0.0;
             if constexpr (PipeState<SOL>::DELAY) qold[m] = S.q_m4[m];
-            else qold[m] = upd ? load_q<MX, MBC, FUSED>(a, T, m, s - 4) : 0.0;
+            else if constexpr (FUSED) qold[m] = upd ? a.qsrc[dst + m * a.strip.nxp * a.strip.nxp] : 0.0;
+            else qold[m] = upd ? T.q[((int64_t)m * NX + s - 4) * NX] : 0.0;
         }
     }
 
@@ -311,7 +276,7 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
         for (int m = 0; m < M; ++m) {
             double gxd = 0.0, gxu = 0.0;
             if (xint) {
-                if (c + 1 <= NX - 1) {
+                if (c + 1 <= NXL - 1) {
                     gxd = -(double)gl[(0 * M + m) * L::PNX + 1] - (double)S.gRmx[m];
                     gxu = -(double)gl[(1 * M + m) * L::PNX + 1] - (double)S.gRpx[m];
                 } else {
@@ -345,7 +310,9 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
             const double* gy = T.db + L::GY + s4(4) * (2 * M * L::PNX);
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                double* qp = T.q + ((int64_t)m * NY + r) * NX;
+                double* qp;
+                if constexpr (FUSED) qp = T.q + dst + m * a.strip.nxp * a.strip.nxp;
+                else qp = T.q + ((int64_t)m * NX + r) * NX;
                 const double fxm1 = fx[(0 * M + m) * L::PNX + 1];  // FP32 flux parts widen exactly
                 const double fxp0 = fx[(1 * M + m) * L::PNX];
                 const double gyu_l = (c >= 1) ? gy[(1 * M + m) * L::PNX - 1] : 0.0;
@@ -436,14 +403,14 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 R am[M], ap[M];
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
-                    R fmv = (c <= NX - 2) ? S.xam[m] : R(0);
+                    R fmv = (c <= NXL - 2) ? S.xam[m] : R(0);
                     R fpv = (c <= NX - 2) ? -S.xap[m] : R(0);
                     if (meth.second_order()) { fmv = fmv + R(0.5) * cq[m]; fpv = fpv + R(0.5) * cq[m]; }
                     fx[(0 * M + m) * L::PNX] = fmv;
                     fx[(1 * M + m) * L::PNX] = fpv;
                     am[m] = S.xam[m];
                     ap[m] = S.xap[m];
-                    if (meth.transverse2() && c <= NX - 2) { am[m] = am[m] + cq[m]; ap[m] = ap[m] - cq[m]; }
+                    if (meth.transverse2() && c <= NXL - 2) { am[m] = am[m] + cq[m]; ap[m] = ap[m] - cq[m]; }
                 }
                 R* gl = T.rb + L::GL + s2(2) * (2 * M * L::PNX);
                 if (meth.transverse()) {
@@ -528,7 +495,7 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
             QT* qr = qb + L::Q + s2(0) * (M * L::PNX);
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                if (T.save_last) T.qlast[((int64_t)m * NY + s) * NX] = S.qcur[m];
+                if (T.save_last) T.qlast[((int64_t)m * NX + s) * NX] = S.qcur[m];
                 qr[m * L::PNX] = QT(S.qcur[m]);
             }
             // raw y-interface s (between rows s-1 and s)
@@ -567,10 +534,10 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
         }
         // clawpack 5: interfaces MBC..MBC+MX carry fluxes; f = MBC+MX+1 only
         // closes the transverse sum of cell row MBC+MX
-        const bool yblk = T.ycol && (R15 ? (f >= MBC && f <= MBC + MX + 1) : (STEADY || (f >= 1 && f <= NY - 1)));
+        const bool yblk = T.ycol && (R15 ? (f >= MBC && f <= MBC + MY + 1) : (STEADY || (f >= 1 && f <= NY - 1)));
         if (yblk) {
-            const bool fact = !R15 || f <= MBC + MX;
-            const bool inner = R15 ? fact : (STEADY || (f >= MBC && f <= MBC + MX));
+            const bool fact = !R15 || f <= MBC + MY;
+            const bool inner = R15 ? fact : (STEADY || (f >= MBC && f <= MBC + MY));
             const bool god = R15 ? fact : (STEADY || f <= NY - 2);
             R w[W][M];
 #pragma unroll
@@ -642,7 +609,7 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 for (int m = 0; m < M; ++m) gLm[m] = gLp[m] = gRm[m] = gRp[m] = R(0);
             }
             // cell row f-1 is complete: gadd(f-1,.,1) = (0 - gL(f)) - gR(f-1)
-            if (R15 ? (f - 1 >= MBC && f - 1 <= MBC + MX) : (STEADY || f - 1 >= 1)) {
+            if (R15 ? (f - 1 >= MBC && f - 1 <= MBC + MY) : (STEADY || f - 1 >= 1)) {
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
                     GYd[m] = -(double)gLm[m] - (double)S.gRm_prev[m];
@@ -709,7 +676,10 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 if (T.active) {
                     QT* ax = qb + L::AX + s4(-1) * (NAUX * L::PNX);
 #pragma unroll
-                    for (int kk = 0; kk < NAUX; ++kk) ax[kk * L::PNX] = QT(T.aux[(kk * NY + s + 1) * NX]);
+                    for (int kk = 0; kk < NAUX; ++kk) {
+                        if constexpr (FUSED) ax[kk * L::PNX] = QT(strip_aux(a, T.xm, T.y0 - 2 + s + 1, kk));
+                        else ax[kk * L::PNX] = QT(T.aux[(kk * NX + s + 1) * NX]);
+                    }
                 }
             }
         }
@@ -733,12 +703,11 @@ constexpr bool pipe_six_ctas() {
     return sizeof(typename SOL::Real) == 4 && SOL::M == 1;
 }
 
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+// NX: columns of a patch, ghost columns included; of a strip (FUSED): the most it has.
+template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
 __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     constexpr int M = SOL::M;
     constexpr int W = SOL::W;
-    constexpr int NX = MX + 2 * MBC;
-    constexpr int NY = NX;
     constexpr bool SWIRL = AUXK == AUX_SWIRL;
     constexpr int TPP = pipe_threads_per_patch<NX, SWIRL>();
     constexpr int PPB = TPB / TPP;
@@ -756,13 +725,26 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     const int pl = t / TPP;
     const int c = t - pl * TPP;
     const int pg = blockIdx.x * PPB + pl;
-    const bool patch_ok = (pl < PPB) && (pg < a.npatches);
-    const bool active = patch_ok && c < NX;
+    // a strip: interior columns [x0, x0 + mxs) and rows [y0, y0 + mys) of the mesh
+    const int sx = FUSED ? blockIdx.x % a.strip.nsx : 0, sy = FUSED ? blockIdx.x / a.strip.nsx : 0;
+    const int x0 = sx * a.strip.w, y0 = sy * a.strip.h;
+    const int mxs = FUSED ? min(a.strip.w, a.strip.n - x0) : NX - 2 * MBC;
+    const int mys = FUSED ? min(a.strip.h, a.strip.n - y0) : NX - 2 * MBC;
+    const int NY = FUSED ? mys + 2 * MBC : NX;
+    const bool patch_ok = FUSED ? pl == 0 && c <= mxs + 2 * MBC : (pl < PPB) && (pg < a.npatches);
+    const bool active = patch_ok && c < mxs + 2 * MBC;
     const int pls = patch_ok ? pl : 0;  // threads without a patch read (never write) patch 0's rows
     const int cc = c < NX ? c : NX - 1;
     const PatchDesc* D = (a.desc && patch_ok) ? a.desc + pg : nullptr;  // mixed-solve launch
-    const int slot = (patch_ok && !a.desc) ? a.slots[pg] : 0;
-    const PatchMeta meta = D ? D->meta : (patch_ok ? a.meta[slot] : PatchMeta{0, 0, 1, 1, 0, 0});
+    int slot = 0;
+    if constexpr (FUSED) slot = __ldg(a.strip.grid);  // every patch has the same cell size
+    else slot = (patch_ok && !a.desc) ? a.slots[pg] : 0;
+    PatchMeta meta = D ? D->meta : (FUSED || patch_ok ? a.meta[slot] : PatchMeta{0, 0, 1, 1, 0, 0});
+    if constexpr (FUSED) {
+        // the strip's own corner: the mesh's cell edges are exact multiples of its spacing
+        meta.xlower = a.strip.ax + (double)x0 * meta.dx;
+        meta.ylower = a.strip.ay + (double)y0 * meta.dy;
+    }
     const int req = D ? D->req : -1;
     SOL sol{R(a.grav), R(a.gamma), R(a.gamma1), R(a.drytol)};
     if constexpr (SOL::FWAVE) {
@@ -775,26 +757,25 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     T.active = active;
     T.node = SWIRL && patch_ok;
     T.save_last = active && (meta.flags & PATCH_SAVE_LAST);
-    T.ycol = active && c >= 1 && c <= NX - 2;
-    T.q = (D ? D->q : a.q + (int64_t)slot * a.q_stride) + cc;
+    T.ycol = active && c >= 1 && c <= mxs + 2 * MBC - 2;
+    T.mx = mxs;
+    T.ny = NY;
+    if constexpr (FUSED) T.q = a.q;
+    else T.q = (D ? D->q : a.q + (int64_t)slot * a.q_stride) + cc;
     T.qlast = (D ? D->qlast : a.qlast + (int64_t)slot * a.q_stride) + cc;
-    T.slot = slot;
-    T.qs = nullptr;
-    T.negmid = 0u;
+    T.x = T.xm = T.y0 = 0;
+    T.negx = 0u;
+    PipeState<SOL> S;
+    S.sslot = S.dslot = 0;
     if constexpr (FUSED) {
-        // rows MBC..MBC+MX-1 of this column come from one place (own patch,
-        // face neighbour, or the own patch's boundary column); rows outside are
-        // resolved row by row in load_q
         T.save_last = false;  // a mesh of one level has no patch with finer neighbours
-        if (active) {
-            const double* p0;
-            unsigned neg;
-            fused_src<MX, MBC>(a, slot, cc, MBC, p0, neg);
-            T.qs = p0 - (int64_t)MBC * NX;
-            T.negmid = neg;
-        }
+        bool wall;
+        T.xm = x0 - MBC + c;
+        T.x = strip_inside(T.xm, a.strip.n, a.strip.bc[0], a.strip.bc[1], wall);
+        T.negx = wall ? 2u : 0u;
+        T.y0 = y0;
     }
-    T.aux = (AUXK == AUX_STORED && active) ? (D ? D->aux : a.aux + (int64_t)slot * a.aux_stride) + cc : nullptr;
+    T.aux = (AUXK == AUX_STORED && active && !FUSED) ? (D ? D->aux : a.aux + (int64_t)slot * a.aux_stride) + cc : nullptr;
     T.rb = rsm + pls * NX + cc;
     T.db = dsm + pls * NX + cc;
     T.nb = dsm + L::ND + pls * (NX + 1) + c;
@@ -820,11 +801,14 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
         }
     }
 
-    PipeState<SOL> S;
+#pragma unroll
+    for (int m = 0; m < M; ++m) S.qcur[m] = S.qpre[m] = 0.0;
+    if (active) {
+        load_row<SOL, NX, FUSED>(a, T, S, 0, S.qcur);
+        load_row<SOL, NX, FUSED>(a, T, S, 1, S.qpre);
+    }
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-        S.qcur[m] = active ? load_q<MX, MBC, FUSED>(a, T, m, 0) : 0.0;
-        S.qpre[m] = active ? load_q<MX, MBC, FUSED>(a, T, m, 1) : 0.0;
         S.q_m1[m] = 0.0;
         S.q_m2[m] = S.q_m3[m] = S.q_m4[m] = 0.0;
         S.yam_f[m] = S.yap_f[m] = R(0);
@@ -860,7 +844,14 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
             const double y = meta.ylower + (double)(c - MBC) * meta.dy;
             const double sx = sin(pi * x), sy = sin(pi * y);
             T.tx = sx * sx;
-            if (T.node) dsm[L::TY + pls * (NX + 1) + c] = sy * sy;
+            if constexpr (FUSED) {
+                for (int k = t; k <= NY; k += TPB) {
+                    const double sk = sin(pi * (meta.ylower + (double)(k - MBC) * meta.dy));
+                    dsm[L::TY + k] = sk * sk;
+                }
+            } else {
+                if (T.node) dsm[L::TY + pls * (NX + 1) + c] = sy * sy;
+            }
         }
         __syncthreads();
         const double p0 = psi_node<R>(T.tx, T.ty[0]), p1 = psi_node<R>(T.tx, T.ty[1]);
@@ -878,8 +869,11 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
         if (active) {
 #pragma unroll
             for (int k = 0; k < NAUX; ++k) {
-                if constexpr (ring_in_fp64<SOL>) T.db[L::AX + k * L::PNX] = T.aux[(k * NY + 0) * NX];
-                else T.rb[L::AX + k * L::PNX] = QT(T.aux[(k * NY + 0) * NX]);
+                double v;
+                if constexpr (FUSED) v = strip_aux(a, T.xm, T.y0 - 2, k);
+                else v = T.aux[k * NX * NX];
+                if constexpr (ring_in_fp64<SOL>) T.db[L::AX + k * L::PNX] = v;
+                else T.rb[L::AX + k * L::PNX] = QT(v);
             }
         }
     }
@@ -887,15 +881,15 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
 
     // ---- rows: ramp-up, steady state (unrolled by the ring period 4), ramp-down ----
     int s = 0;
-    for (; s < 4; ++s) pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, -1, false, FUSED>(a, sol, T, S, s);
-    constexpr int NSTEADY = NY - 5;  // s = 4 .. NY-2
+    for (; s < 4; ++s) pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, -1, false, FUSED>(a, sol, T, S, s);
+    const int NSTEADY = NY - 5;  // s = 4 .. NY-2
     for (int rnd = 0; rnd < NSTEADY / 4; ++rnd, s += 4) {
-        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 0, true, FUSED>(a, sol, T, S, s);
-        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 1, true, FUSED>(a, sol, T, S, s + 1);
-        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 2, true, FUSED>(a, sol, T, S, s + 2);
-        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 3, true, FUSED>(a, sol, T, S, s + 3);
+        pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, 0, true, FUSED>(a, sol, T, S, s);
+        pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, 1, true, FUSED>(a, sol, T, S, s + 1);
+        pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, 2, true, FUSED>(a, sol, T, S, s + 2);
+        pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, 3, true, FUSED>(a, sol, T, S, s + 3);
     }
-    for (; s <= NY + 2; ++s) pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, -1, false, FUSED>(a, sol, T, S, s);
+    for (; s <= NY + 2; ++s) pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, -1, false, FUSED>(a, sol, T, S, s);
 
     // ---- CFL: warp max, one atomic per warp ----
     // flux2: cfl = max(cfl, dtdx*s, -dtdx*s) over the interfaces.  Rounding is
@@ -919,21 +913,21 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     }
 }
 
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
 __global__ void __launch_bounds__(TPB) step_kernel_pipe(const StepArgs a) {
-    step_pipe_body<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>(a);
+    step_pipe_body<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>(a);
 }
 
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
 __global__ void __launch_bounds__(TPB, 6) step_kernel_pipe_six(const StepArgs a) {
-    step_pipe_body<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>(a);
+    step_pipe_body<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>(a);
 }
 
 // the one kernel of the two that a form uses (only that one is instantiated)
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
 constexpr auto pipe_kernel() {
-    if constexpr (pipe_six_ctas<SOL>()) return step_kernel_pipe_six<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>;
-    else return step_kernel_pipe<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>;
+    if constexpr (pipe_six_ctas<SOL>()) return step_kernel_pipe_six<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>;
+    else return step_kernel_pipe<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>;
 }
 
 // ---------------------------------------------------------------------------
@@ -941,24 +935,45 @@ constexpr auto pipe_kernel() {
 // ---------------------------------------------------------------------------
 namespace {
 
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
 cudaError_t launch_pipe_one(const StepArgs& a, cudaStream_t st) {
-    constexpr int NX = MX + 2 * MBC;
     constexpr int PPB = TPB / pipe_threads_per_patch<NX, AUXK == AUX_SWIRL>();
     static_assert(PPB >= 1, "patch wider than the CTA");
     using L = PipeSmem<NX, PPB, SOL::M, SOL::W, NAUX, AUXK == AUX_SWIRL, typename SOL::Real, ring_in_fp64<SOL>>;
-    const size_t bytes = (size_t)L::BYTES;
-    constexpr auto kernel = pipe_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>();
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return e;
-        configured = true;
+    constexpr auto kernel = pipe_kernel<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>();
+    if constexpr (!FUSED) {
+        const size_t bytes = (size_t)L::BYTES;
+        static bool configured = false;
+        if (!configured) {
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            if (e != cudaSuccess) return e;
+            configured = true;
+        }
+        const int blocks = (a.npatches + PPB - 1) / PPB;
+        if (blocks == 0) return cudaSuccess;
+        kernel<<<blocks, TPB, bytes, st>>>(a);
+        return cudaGetLastError();
+    } else {
+        // bytes of a strip of h rows: its table of node rows replaces the patches'
+        constexpr bool SWIRL = AUXK == AUX_SWIRL;
+        auto bytes_of = [](int h) { return (int)(L::BYTES + (SWIRL ? (h + 2 * MBC + 1 - L::NDS) * 8 : 0)); };
+        static std::atomic<int> per_wave{0};
+        if (per_wave.load() == 0) {
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 bytes_of(kStripRowsMax));
+            if (e != cudaSuccess) return e;
+            int dev = 0, sms = 0, occ = 0;
+            if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+            if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, TPB, bytes_of(256))) != cudaSuccess)
+                return e;
+            per_wave.store(std::max(1, sms * occ));
+        }
+        StepArgs b = a;
+        strip_plan(b.strip, NX - 2 * MBC, per_wave.load());
+        kernel<<<b.strip.nsx * b.strip.nsy, TPB, bytes_of(b.strip.h), st>>>(b);
+        return cudaGetLastError();
     }
-    const int blocks = (a.npatches + PPB - 1) / PPB;
-    if (blocks == 0) return cudaSuccess;
-    kernel<<<blocks, TPB, bytes, st>>>(a);
-    return cudaGetLastError();
 }
 
 // Limiter specialisation: every wave limited with the same code and order (2, 2).
@@ -971,23 +986,29 @@ int fixed_limiter(const StepArgs& a) {
     return (l == 3 || l == 4) ? l : 0;
 }
 
-template <class SOL, int MX, int AUXK, int NAUX, bool FUSED>
+template <class SOL, int NX, int AUXK, int NAUX, bool FUSED>
 cudaError_t launch_pipe_lim(const StepArgs& a, cudaStream_t st) {
     switch (fixed_limiter<SOL>(a)) {
-        case 3: return launch_pipe_one<SOL, MX, 2, AUXK, NAUX, 128, 3, FUSED>(a, st);
-        case 4: return launch_pipe_one<SOL, MX, 2, AUXK, NAUX, 128, 4, FUSED>(a, st);
-        default: return launch_pipe_one<SOL, MX, 2, AUXK, NAUX, 128, 0, FUSED>(a, st);
+        case 3: return launch_pipe_one<SOL, NX, 2, AUXK, NAUX, 128, 3, FUSED>(a, st);
+        case 4: return launch_pipe_one<SOL, NX, 2, AUXK, NAUX, 128, 4, FUSED>(a, st);
+        default: return launch_pipe_one<SOL, NX, 2, AUXK, NAUX, 128, 0, FUSED>(a, st);
     }
 }
 
 template <class SOL, int AUXK, int NAUX, bool FUSED>
 cudaError_t launch_pipe_mx(int mx, int mbc, const StepArgs& a, cudaStream_t st) {
     if (mbc != 2) return cudaErrorNotSupported;
-    switch (mx) {
-        case 8: return launch_pipe_lim<SOL, 8, AUXK, NAUX, FUSED>(a, st);
-        case 16: return launch_pipe_lim<SOL, 16, AUXK, NAUX, FUSED>(a, st);
-        case 32: return launch_pipe_lim<SOL, 32, AUXK, NAUX, FUSED>(a, st);
-        default: return cudaErrorNotSupported;
+    if constexpr (FUSED) {
+        // strips take patches of any size; with the swirl velocities the last
+        // thread of the CTA works on a node column alone
+        return launch_pipe_lim<SOL, AUXK == AUX_SWIRL ? 127 : 128, AUXK, NAUX, true>(a, st);
+    } else {
+        switch (mx) {
+            case 8: return launch_pipe_lim<SOL, 12, AUXK, NAUX, false>(a, st);
+            case 16: return launch_pipe_lim<SOL, 20, AUXK, NAUX, false>(a, st);
+            case 32: return launch_pipe_lim<SOL, 36, AUXK, NAUX, false>(a, st);
+            default: return cudaErrorNotSupported;
+        }
     }
 }
 
@@ -1009,19 +1030,16 @@ cudaError_t launch_step_pipe_v(int solver, int aux_kind, int mwaves, int mx, int
             return cudaErrorNotSupported;
         case SOLVER_SWE_ROE:
             if (mwaves != 3 || aux_kind != AUX_NONE) return cudaErrorNotSupported;
-            if constexpr (FUSED) return launch_pipe_mx<SweRoeT<R, V5>, AUX_NONE, 0, FUSED>(mx, mbc, a, st);
             break;
         case SOLVER_EULER4_ROE:
             if (mwaves != 4 || aux_kind != AUX_NONE) return cudaErrorNotSupported;
-            if constexpr (FUSED) return launch_pipe_mx<Euler4RoeT<R, V5>, AUX_NONE, 0, FUSED>(mx, mbc, a, st);
             break;
         case SOLVER_GEOCLAW_FWAVE:
             if (V5 || mwaves != 3 || aux_kind != AUX_STORED || a.maux != 1) return cudaErrorNotSupported;
-            if constexpr (FUSED && !V5) return launch_pipe_mx<GeoclawFwaveT<R>, AUX_STORED, 1, FUSED>(mx, mbc, a, st);
             break;
         default: return cudaErrorNotSupported;
     }
-    // the unfused systems: both sweeps of a column on two threads
+    // the systems: both sweeps of a column on two threads, patches or strips
     if (mbc != 2) return cudaErrorNotSupported;
     if constexpr (std::is_same_v<R, float>) return launch_split_mixed(solver, mx, V5 ? 5 : 4, a, st);
     else if (solver == SOLVER_SWE_ROE) return launch_split_swe(mx, V5 ? 5 : 4, a, st);
@@ -1029,11 +1047,11 @@ cudaError_t launch_step_pipe_v(int solver, int aux_kind, int mwaves, int mx, int
     else return launch_split_geoclaw(mx, a, st);
 }
 
-// FUSED: the ghost-exchange-fused form (a.fuse and a.qsrc set; mesh of one level)
+// FUSED: the ghost-exchange-fused form (a.strip and a.qsrc set; mesh of one level)
 template <typename R, bool FUSED>
 cudaError_t launch_step_pipe_t(int solver, int aux_kind, int mwaves, int mx, int my, int mbc, int claw_version,
                                const StepArgs& a, cudaStream_t st) {
-    if (FUSED != (a.fuse != nullptr) || (FUSED && (a.desc || !a.qsrc || a.qsrc == a.q))) return cudaErrorInvalidValue;
+    if (FUSED != (a.strip.grid != nullptr) || (FUSED && (a.desc || !a.qsrc || a.qsrc == a.q))) return cudaErrorInvalidValue;
     if (claw_version == 5) return launch_step_pipe_v<R, true, FUSED>(solver, aux_kind, mwaves, mx, my, mbc, a, st);
     return launch_step_pipe_v<R, false, FUSED>(solver, aux_kind, mwaves, mx, my, mbc, a, st);
 }
