@@ -800,18 +800,139 @@ struct GeoclawFwaveT {
     struct Roe { R s[3]; };  // the wave speeds: no Roe averages, there is no transverse solver
     struct Cell {};
     static constexpr int NC = 0;
-    static constexpr int NWV = 9;
-    __host__ __device__ static constexpr bool nz(int, int) { return true; }
+    // wave components that are not zero by construction: the middle wave moves
+    // momentum in the normal direction alone
+    static constexpr int NWV = 7;
+    __host__ __device__ static constexpr bool nz(int mw, int rel) { return mw != 1 || rel == 1; }
     __device__ __forceinline__ void speeds(const Roe& rr, R* s) const {
         s[0] = rr.s[0];
         s[1] = rr.s[1];
         s[2] = rr.s[2];
     }
     R grav, gamma, gamma1, drytol;
-    // one interface of rpn2_geoclaw.f90; the states and bL, bR (aux(1) of the
-    // two cells) in FP64
+    // The common interface (both sides wet, subcritical) without a branch per
+    // division (fcb_arith.cuh): the eigenvectors' zeros and ones multiplied out, the
+    // sign tests that bound deldelh made on products with a margin of 0.1 %.  Every
+    // other interface, and operands near underflow, take rpn2b_plain.
     __device__ __forceinline__ void rpn2b(int ixy, const double* qL, const double* qR, double bL, double bR,
                                           R (*wave)[M], R* s, R* amdq, R* apdq, bool& bad) const {
+        const int mu = (ixy == 1) ? 1 : 2;
+        const int mv = (ixy == 1) ? 2 : 1;
+        const double g = gdbl, dtol = drytol_d;
+        const double hL = qL[0], hR = qR[0], huL = qL[mu], huR = qR[mu];
+        bool ok = hL > dtol && hR > dtol;
+        const Dv<double> dL(hL, ok), dR(hR, ok);
+        const double uL = dL(huL, ok), vL = dL(qL[mv], ok), phiL = 0.5 * g * (hL * hL) + dL(huL * huL, ok);
+        const double uR = dR(huR, ok), vR = dR(qR[mv], ok), phiR = 0.5 * g * (hR * hR) + dR(huR * huR, ok);
+        const double cL = sqrt_ok(g * hL, ok), cR = sqrt_ok(g * hR, ok);
+        const R rg = R(g), ruL = R(uL), ruR = R(uR), rhL = R(hL), rhR = R(hR);
+        R rcL, rcR;
+        if constexpr (sizeof(R) == 8) { rcL = cL; rcR = cR; }
+        else { rcL = sqrt(rg * rhL); rcR = sqrt(rg * rhR); }
+        const R uhat = Dv<R>(rcR + rcL, ok)(rcL * ruL + rcR * ruR, ok);
+        const R chat = sqrt_ok(rg * R(0.5) * (rhR + rhL), ok);
+        R sE1 = dmin(ruL - rcL, uhat - chat), sE2 = dmax(ruR + rcR, uhat + chat);
+        // riemanntype, both sides wet: the speeds of the middle state's outer waves
+        R s1m, s2m;
+        {
+            const R delu = ruR - ruL;
+            const bool leftmin = rhL < rhR;
+            const R hmin = leftmin ? rhL : rhR, hmax = leftmin ? rhR : rhL;
+            const R cmin = leftmin ? rcL : rcR, cmax = leftmin ? rcR : rcL;
+            const R fmin_ = delu + R(2.0) * (cmin - cmax);
+            const R fmax_ = delu + (hmax - hmin) * sqrt_ok(Dv<R>(hmax * hmin, ok)(R(.5) * rg * (hmax + hmin), ok), ok);
+            if (fmin_ <= R(0.0) && fmax_ <= R(0.0)) {  // two shocks
+                const Dv<R> d0(hmax, ok), l(rhL, ok), r(rhR, ok);
+                const R i0 = d0(R(1), ok), iL = l(R(1), ok), iR = r(R(1), ok);
+                const R gL = sqrt_ok(R(.5) * rg * (i0 + iL), ok), gR = sqrt_ok(R(.5) * rg * (i0 + iR), ok);
+                const R F0 = delu + (hmax - rhL) * gL + (hmax - rhR) * gR;
+                const R hh = R(4.0) * (hmax * hmax);
+                const R dfdh = gL - Dv<R>(hh * gL, ok)(rg * (hmax - rhL), ok) + gR -
+                               Dv<R>(hh * gR, ok)(rg * (hmax - rhR), ok);
+                const R sq0 = sqrt_ok(hmax, ok);
+                const R slope = R(2.0) * sq0 * dfdh;
+                const R t = sq0 - Dv<R>(slope, ok)(F0, ok);
+                const R hm = t * t;
+                const R im = Dv<R>(hm, ok)(R(1), ok), cm = sqrt_ok(rg * hm, ok);
+                s1m = ruL - (hm - rhL) * sqrt_ok((R(.5) * rg) * (im + iL), ok) - cm;
+                s2m = ruR + (hm - rhR) * sqrt_ok((R(.5) * rg) * (im + iR), ok) + cm;
+            } else {
+                const bool rare = fmin_ > R(0.0);  // two rarefactions, else a shock and a rarefaction
+                // (a shock and a rarefaction: F0 at h_min is fmin_, a zero added)
+                const R slope = Dv<R>(rare ? R(1) : hmax - hmin, ok)(rare ? R(1) : fmax_ - fmin_, ok);
+                const R step = Dv<R>(slope, ok)(rare ? R(0) : -fmin_, ok);  // fmin_ <= 0 here
+                const R t = dmax(R(0.0), -delu + R(2.0) * (rcL + rcR));
+                const R i16 = Dv<R>(R(16.0) * rg, ok)(R(1), ok);
+                const R hm = rare ? i16 * (t * t) : hmin + step;
+                const R cm = sqrt_ok(rg * hm, ok);
+                const R ul = ruL + R(2.0) * rcL, ur = ruR - R(2.0) * rcR;
+                const bool left = rhL > rhR;
+                s1m = rare || left ? ul - R(3.0) * cm : ur + cm;
+                s2m = rare || !left ? ur + R(3.0) * cm : ul - cm;
+            }
+        }
+        const R l0 = dmin(sE1, s2m), l2 = dmax(sE2, s1m), l1 = R(0.5) * (l0 + l2);
+        const Dv<R> dl(l2 - l0, ok);  // sE2 - sE1, and minus the determinant
+        const R hstarHLL = dmax(dl(R(huL) - R(huR) + l2 * rhR - l0 * rhL, ok), R(0.0));
+        const double ctol = dmax(dtol * g, 1e-6);
+        const double hbar = dmax(0.5 * (hL + hR), 0.0);
+        const double s1s2bar = 0.25 * ((uL + uR) * (uL + uR)) - g * hbar;
+        const double s1s2tilde = dmax(0.0, uL * uR) - g * hbar;
+        const double dE1 = l0, dE2 = l2;
+        bool sonic = false;
+        if (fabs(s1s2bar) <= ctol) sonic = true;
+        if (s1s2bar * s1s2tilde <= ctol * ctol) sonic = true;
+        if (s1s2bar * dE1 * dE2 <= ctol * ctol) sonic = true;
+        if (dmin(fabs(dE1), fabs(dE2)) < ctol2) sonic = true;
+        if (dE1 < ctol2 && (double)s1m > -ctol2) sonic = true;
+        if (dE2 > -ctol2 && (double)s2m < ctol2) sonic = true;
+        if ((uL + cL) * (uR + cR) < 0.0) sonic = true;
+        if ((uL - cL) * (uR - cR) < 0.0) sonic = true;
+        const double delb = bR - bL, w = delb * g * hbar;
+        const Dv<double> dbar(-s1s2bar, ok);  // subcritical: negative
+        const double deldelh = -dbar(w, ok);
+        // deldelh stays inside [HLL / sE1, HLL / sE2]
+        const double hll = (double)(hstarHLL * (l2 - l0));
+        ok = ok && dE1 < -ctol && dE2 > ctol && hll > 0.0 && deldelh * dE2 < 0.999 * hll && deldelh * dE1 < 0.999 * hll;
+        double deldelphi = dbar(w * s1s2tilde, ok);
+        deldelphi = dmin(deldelphi, g * dmax(-hL * delb, -hR * delb));
+        deldelphi = dmax(deldelphi, g * dmin(-hL * delb, -hR * delb));
+        const R d0 = R((hR - hL) - deldelh), d1 = R(huR - huL), d2 = R((phiR - phiL) - deldelphi);
+        const R q0 = l0 * l0, q2 = l2 * l2;
+        const R b0 = -dl(d0 * -l2 + d1, ok), b2 = -dl(-d1 + d0 * l0, ok);
+        const R b1 = -dl((d1 * q2 - l2 * d2) - d0 * (l0 * q2 - l2 * q0) + (l0 * d2 - d1 * q0), ok);
+        R f0 = b0 * l0 * R(vL), f2 = b2 * l2 * R(vR);
+        const R dvflux = R(hR * uR * vR - hL * uL * vL), rest = dvflux - f0 - f2;
+        if (huL + (double)(b0 * l0) <= 0.0) f0 = f0 + rest;
+        else f2 = f2 + rest;
+        s[0] = l0; s[1] = l1; s[2] = l2;
+        wave[0][0] = b0 * l0; wave[0][mu] = b0 * q0; wave[0][mv] = f0;
+        wave[1][0] = R(0.0); wave[1][mu] = b1; wave[1][mv] = R(0.0);
+        wave[2][0] = b2 * l2; wave[2][mu] = b2 * q2; wave[2][mv] = f2;
+        if (!ok) {
+            seldom();
+            rpn2b_plain(ixy, qL, qR, bL, bR, wave, s, bad);
+        } else if (sonic) {
+            bad = true;
+        }
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            R am = R(0.0), ap = R(0.0);
+#pragma unroll
+            for (int mw = 0; mw < 3; ++mw) {
+                if (mw == 1 && m != mu) continue;  // zero
+                const R half = R(0.5) * wave[mw][m];
+                am = am + (s[mw] < R(0.0) ? wave[mw][m] : s[mw] > R(0.0) ? R(0.0) : half);
+                ap = ap + (s[mw] > R(0.0) ? wave[mw][m] : s[mw] < R(0.0) ? R(0.0) : half);
+            }
+            amdq[m] = am;
+            apdq[m] = ap;
+        }
+    }
+    // one interface of rpn2_geoclaw.f90; the states and bL, bR (aux(1) of the
+    // two cells) in FP64
+    __device__ __forceinline__ void rpn2b_plain(int ixy, const double* qL, const double* qR, double bL, double bR,
+                                                R (*wave)[M], R* s, bool& bad) const {
         const int mu = (ixy == 1) ? 1 : 2;
         const int mv = (ixy == 1) ? 2 : 1;
         // the FP64 hydrostatic part reads gravity and the dry tolerance in FP64
@@ -875,23 +996,9 @@ struct GeoclawFwaveT {
                 wave[mw][mv] = fw[2][mw] * wall[mw];
             }
         }
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-            R am = R(0.0), ap = R(0.0);
-#pragma unroll
-            for (int mw = 0; mw < 3; ++mw) {
-                if (s[mw] < R(0.0)) am = am + wave[mw][m];
-                else if (s[mw] > R(0.0)) ap = ap + wave[mw][m];
-                else {
-                    am = am + R(0.5) * wave[mw][m];
-                    ap = ap + R(0.5) * wave[mw][m];
-                }
-            }
-            amdq[m] = am;
-            apdq[m] = ap;
-        }
     }
     double gdbl, drytol_d;  // gravity and dry tolerance in FP64, set by the step kernel
+    double ctol2;           // the root of the critical tolerance, likewise
     // never called: order (2, 0) is enforced for this solver
     __device__ __forceinline__ void rpt2(int, const R* asdq, const Roe&, R, R, R* bm, R* bp) const {
 #pragma unroll

@@ -750,6 +750,7 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     if constexpr (SOL::FWAVE) {
         sol.gdbl = a.grav;
         sol.drytol_d = a.drytol;
+        sol.ctol2 = sqrt(dmax(a.drytol * a.grav, 1e-6));
     }
 
     PipeThread<R> T;

@@ -27,7 +27,7 @@
 // counters are uniform.  Shallow water, mx = 32, 1,024 patches, one level update on
 // B200: 0.395 ms in the four-barrier form, 0.139 ms here (FP64 pipe 46 %, issue slots
 // 60 %; stalls: fixed latencies and the barrier); Euler, mx = 16, 4,096 patches: 0.856
-// and 0.320 ms; GeoClaw, mx = 32, 1,024 patches: 0.324 ms (pipelined form of one thread
+// and 0.320 ms; GeoClaw, mx = 32, 1,024 patches: 0.157 ms (pipelined form of one thread
 // per column: 0.57 ms).
 //
 // Arithmetic, operation order and loop bounds are those of the reference
@@ -100,7 +100,9 @@ struct SplitSmem {
     static constexpr bool KEEPX = TR && sizeof(R) == 8 && M == 3, KEEPY = TR && sizeof(R) == 8;
     static constexpr int KX = AX + (QD ? 0 : 3 * NAUX * PNX);     // 2M
     static constexpr int KY = KX + (KEEPX ? 2 * M * PNX : 0);     // 2M
-    static constexpr int NR = KY + (KEEPY ? 2 * M * PNX : 0);
+    // the f-waves of the y-interface that is final next
+    static constexpr int KW = KY + (KEEPY ? 2 * M * PNX : 0);     // W*M
+    static constexpr int NR = KW + (SOL::FWAVE ? SOL::NWV * PNX : 0);
     static constexpr int BYTES = ND * 8 + ((NR * (int)sizeof(R) + 15) / 16) * 16;
 };
 
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(2 * HALF) step_kernel_split(const StepArgs a) 
     if constexpr (FWAVE) {
         sol.gdbl = a.grav;
         sol.drytol_d = a.drytol;
+        sol.ctol2 = sqrt(dmax(a.drytol * a.grav, 1e-6));
     }
     double pdt, pdx, pdy;
     bool save_last;
@@ -211,16 +214,15 @@ __global__ void __launch_bounds__(2 * HALF) step_kernel_split(const StepArgs a) 
         // products of its waves with those of f-1
         typename SOL::Roe yR{};
         R yam[M], yap[M], ydotl[W], gRm_prev[M], gRp_prev[M];  // gR: transverse parts into row f-1 (KEEPY: in shared memory)
-        R yw[FWAVE ? W : 1][M];  // f-waves: the waves themselves
 #pragma unroll
         for (int m = 0; m < M; ++m) yam[m] = yap[m] = gRm_prev[m] = gRp_prev[m] = R(0);
 #pragma unroll
         for (int mw = 0; mw < W; ++mw) ydotl[mw] = R(0);
         if constexpr (FWAVE) {
+            if (active) {
 #pragma unroll
-            for (int mw = 0; mw < W; ++mw)
-#pragma unroll
-                for (int m = 0; m < M; ++m) yw[mw][m] = R(0);
+                for (int k = 0; k < SOL::NWV; ++k) rb[L::KW + k * PNX] = R(0);
+            }
         }
         // address of row `row`, component 0, and the components a wall negates; strip:
         // rows come in order, the slot is looked up again at patch edges and outside
@@ -303,11 +305,12 @@ __global__ void __launch_bounds__(2 * HALF) step_kernel_split(const StepArgs a) 
             for (int mw = 0; mw < W; ++mw) ydotr[mw] = R(0);
             if constexpr (FWAVE) {
                 sol.speeds(yR, ysp);
+                int w0 = 0;
 #pragma unroll
                 for (int mw = 0; mw < W; ++mw)
 #pragma unroll
                     for (int m = 0; m < M; ++m) {
-                        w[mw][m] = yw[mw][m];
+                        if (SOL::nz(mw, wave_rel(2, m))) w[mw][m] = rb[L::KW + (w0++) * PNX];
                         wn[mw][m] = R(0);
                     }
             } else {
@@ -495,10 +498,15 @@ __global__ void __launch_bounds__(2 * HALF) step_kernel_split(const StepArgs a) 
                 for (int m = 0; m < M; ++m) yam[m] = yap[m] = R(0);
             }
             if constexpr (FWAVE) {
+                int w0 = 0;
 #pragma unroll
                 for (int mw = 0; mw < W; ++mw)
 #pragma unroll
-                    for (int m = 0; m < M; ++m) yw[mw][m] = wn[mw][m];
+                    for (int m = 0; m < M; ++m)
+                        if (SOL::nz(mw, wave_rel(2, m))) {
+                            if (active) rb[L::KW + w0 * PNX] = wn[mw][m];
+                            ++w0;
+                        }
             }
             // ---- row s and its cell quantities ----
             if (ld) {
@@ -910,10 +918,9 @@ constexpr int split_half() {
 template <class SOL, int MXP, int NAUX, bool TSYNC>
 cudaError_t launch_split_lim(const StepArgs& a, cudaStream_t st) {
     constexpr int HALF = split_half<SOL>();
-    bool mc = a.order0 == 2 && a.order1 == 2;
+    bool mc = a.order0 == 2 && (SOL::FWAVE || a.order1 == 2);  // the f-wave solver has no transverse parts
     for (int mw = 0; mw < SOL::W; ++mw) mc = mc && a.mthlim[mw] == 4;
-    if constexpr (!SOL::FWAVE)
-        if (mc) return launch_split_one<SOL, MXP, NAUX, HALF, 4, TSYNC>(a, st);
+    if (mc) return launch_split_one<SOL, MXP, NAUX, HALF, 4, TSYNC>(a, st);
     return launch_split_one<SOL, MXP, NAUX, HALF, 0, TSYNC>(a, st);
 }
 
