@@ -48,8 +48,8 @@ SOURCES = {
     "fcb_step_split_swe.cu": ["-fmad=false"],
     "fcb_step_split_euler.cu": ["-fmad=false"],
     "fcb_step_split_mixed.cu": ["--use_fast_math"],
-    "fcb_step_fused.cu": ["-fmad=false"],
-    "fcb_step_fused_mixed.cu": ["--use_fast_math"],
+    "fcb_step_adv.cu": ["-fmad=false"],
+    "fcb_step_adv_mixed.cu": ["--use_fast_math"],
     "fcb_ghost.cu": ["-fmad=false"],
     "fcb_amr.cu": ["-fmad=false"],
     "fcb_runtime.cu": [],

@@ -2056,9 +2056,9 @@ void Context::launch_fused_step(double t, double dt, const double* src, double* 
     a.slots = d_level_slots_.p + b;
     a.npatches = e - b;
     cudaError_t r = opt_.precision == 1
-                        ? launch_step_pipe_fused_mixed(opt_.solver_kind, aux_kind_, opt_.mwaves, opt_.mx, opt_.my,
+                        ? launch_step_pipe_mixed(opt_.solver_kind, aux_kind_, opt_.mwaves, opt_.mx, opt_.my,
                                                        opt_.mbc, opt_.claw_version, a, st_)
-                        : launch_step_pipe_fused(opt_.solver_kind, aux_kind_, opt_.mwaves, opt_.mx, opt_.my,
+                        : launch_step_pipe(opt_.solver_kind, aux_kind_, opt_.mwaves, opt_.mx, opt_.my,
                                                  opt_.mbc, opt_.claw_version, a, st_);
     check(r, "fused step");
     cnt_.count_single_step += e - b;

@@ -38,11 +38,7 @@ cudaError_t launch_step_pipe(int solver, int aux_kind, int mwaves, int mx, int m
                              const StepArgs& a, cudaStream_t st);
 cudaError_t launch_step_pipe_mixed(int solver, int aux_kind, int mwaves, int mx, int my, int mbc,
                                    int claw_version, const StepArgs& a, cudaStream_t st);
-// the ghost-exchange-fused pipelined forms (a.strip, a.qsrc set; a mesh of one level)
-cudaError_t launch_step_pipe_fused(int solver, int aux_kind, int mwaves, int mx, int my, int mbc, int claw_version,
-                                   const StepArgs& a, cudaStream_t st);
-cudaError_t launch_step_pipe_fused_mixed(int solver, int aux_kind, int mwaves, int mx, int my, int mbc,
-                                         int claw_version, const StepArgs& a, cudaStream_t st);
+// (a.strip and a.qsrc set: the ghost-exchange-fused form of a mesh of one level)
 // src2 after the step (fcb_src.cu): kind 1 = the axisymmetric Euler source
 cudaError_t launch_src2(int kind, const StepArgs& a, int mx, int my, int mbc, int meqn, cudaStream_t st);
 struct GhostArgs;

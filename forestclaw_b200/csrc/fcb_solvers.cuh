@@ -1027,11 +1027,22 @@ __device__ __forceinline__ R limiter_phi(int mth, R r) {
     }
 }
 
+// num / wn2, wn2 > 0.  The tails of a front leave waves of 1e-136 and less over whole
+// strips of a mesh, whose squares and products are near underflow: both operands
+// times 2^400 (exact) stay in the range of the method.
+__device__ __forceinline__ double limiter_ratio(double num, double wn2, bool& ok) {
+    const double r = Dv<double>(wn2 * 0x1p400, ok, 1400u).quotient(num * 0x1p400);
+    const unsigned h = (unsigned)__double2hiint(r);
+    ok = ok & (h + h - 2u >= (46u << 20) - 2u);  // zero, or |r| >= 2^-1000: not rounded to a denormal
+    return r;
+}
+__device__ __forceinline__ float limiter_ratio(float num, float wn2, bool&) { return num / wn2; }
+
 // Limiter values of the W waves of an interface: phi(num / wn2) for limiter code
 // lim(mw), 1 where the wave vanishes or is not limited.  The quotients are formed
-// together (fcb_arith.cuh), and again with the operator when one of them leaves
-// the range of that method (a wave of 1e-136 and less).  Where the state is
-// constant, whole warps have no wave and skip all of it.
+// together (fcb_arith.cuh), and again with the operator when one of them leaves the
+// range of that method.  Where the state is constant, whole warps have no wave and
+// skip all of it.
 template <bool V5, int W, typename R, class LIM>
 __device__ __forceinline__ void limiter_values(const R* num, const R* wn2, const LIM& lim, R* phi) {
     bool any = false;
@@ -1045,8 +1056,7 @@ __device__ __forceinline__ void limiter_values(const R* num, const R* wn2, const
         R r[W];
 #pragma unroll
         for (int mw = 0; mw < W; ++mw) {
-            const Dv<R> d(wn2[mw] == R(0) ? R(1) : wn2[mw], ok);
-            r[mw] = d(num[mw], ok);
+            r[mw] = limiter_ratio(num[mw], wn2[mw] == R(0) ? R(1) : wn2[mw], ok);
         }
         if (!ok) {
             seldom();

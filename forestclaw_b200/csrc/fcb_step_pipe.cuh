@@ -25,6 +25,9 @@
 // Accumulation order (identical to fcb_step.cu):
 //   fm(i,j) = (FXm + GYu[col i-1]) + GYd[col i],   gm(i,j) = (GXu[row j-1] + GXd[row j]) + FYm
 //   q = q - dtdx*(fm(i+1,j) - fp(i,j)) - dtdy*(gm(i,j+1) - gp(i,j)).
+// It serves scalar advection on meshes of several levels, served and partitioned
+// solves and level calls; the systems run fcb_step_split.cuh, meshes of one level
+// fcb_step_adv.cuh.
 // The kernel is a template on the compute type R of the Riemann solves,
 // limiters and transverse parts (SOL::Real): R = double is the FP64 form,
 // compiled without FMA contraction (fcb_step_pipe.cu); R = float is the mixed
@@ -33,13 +36,10 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include <algorithm>
-#include <atomic>
 #include <type_traits>
 
 #include "fcb_device.h"
 #include "fcb_solvers.cuh"
-#include "fcb_strip.cuh"
 
 namespace fcb {
 
@@ -48,6 +48,9 @@ cudaError_t launch_split_swe(int mx, int claw_version, const StepArgs& a, cudaSt
 cudaError_t launch_split_geoclaw(int mx, const StepArgs& a, cudaStream_t st);
 cudaError_t launch_split_euler(int mx, int claw_version, const StepArgs& a, cudaStream_t st);
 cudaError_t launch_split_mixed(int solver, int mx, int claw_version, const StepArgs& a, cudaStream_t st);
+// scalar advection on a mesh of one level (fcb_step_adv.cuh)
+cudaError_t launch_step_adv(int aux_kind, int claw_version, const StepArgs& a, cudaStream_t st);
+cudaError_t launch_step_adv_mixed(int aux_kind, int claw_version, const StepArgs& a, cudaStream_t st);
 
 namespace {
 
@@ -76,36 +79,26 @@ __device__ __forceinline__ double psi_node(double tx, double ty) {
     else return (tx * ty) * (1.0 / pi);
 }
 
-// Type of the state and aux rings: the compute type, except for the f-wave
-// solver, whose hydrostatic part reads FP64 states and bathymetry; in its mixed
-// form those two rings live in the FP64 region.
-template <class SOL>
-using ring_t = std::conditional_t<SOL::FWAVE, double, typename SOL::Real>;
-template <class SOL>
-constexpr bool ring_in_fp64 = SOL::FWAVE && !std::is_same_v<typename SOL::Real, double>;
-
-template <int NX, int PPB, int M, int W, int NAUX, bool SWIRL, typename R, bool QDBL = false>
+template <int NX, int PPB, int M, int W, int NAUX, bool SWIRL, typename R>
 struct PipeSmem {
     // Rings are [slot][component][patch][column]: one thread's element of any
     // ring sits at (pl * NX + c) + a compile-time offset.
     static constexpr int PNX = PPB * NX;
-    // rings in the compute type R (offsets in R elements); with QDBL the state
-    // (Q) and aux (AX) rings are in the FP64 region instead
-    static constexpr int XW = QDBL ? 0 : 2 * M * PNX; // 2 slots x W*M (after Q: 2 slots x M)
+    // rings in the compute type R (offsets in R elements)
+    static constexpr int Q = 0;                       // 2 slots x M
+    static constexpr int XW = 2 * M * PNX;            // 2 slots x W*M
     static constexpr int GL = XW + 2 * W * M * PNX;   // 2 slots x 2M
     static constexpr int FX = GL + 2 * 2 * M * PNX;   // 4 slots x 2M
-    static constexpr int AXR = FX + 4 * 2 * M * PNX;  // 4 slots x NAUX
-    static constexpr int NR = QDBL ? AXR : AXR + 4 * NAUX * PNX;
+    static constexpr int AX = FX + 4 * 2 * M * PNX;   // 4 slots x NAUX
+    static constexpr int NR = AX + 4 * NAUX * PNX;
     // FP64 region, from byte DBYTES on (offsets in doubles)
     static constexpr int DBYTES = ((NR * (int)sizeof(R) + 15) / 16) * 16;
     static constexpr int GY = 0;                      // 4 slots x 2M: y transverse sums
     static constexpr int NDS = PPB * (NX + 1);
     static constexpr int ND = GY + 4 * 2 * M * PNX;         // swirl: psi node rows, 2 slots [patch][NX+1]
-    static constexpr int TY = ND + (SWIRL ? 2 * NDS : 0);   // swirl: sin^2 of the node rows [patch][NX+1]; last,
-    static constexpr int NDEND = TY + (SWIRL ? NDS : 0);    // since a strip's has its rows + 1 entries instead
-    static constexpr int Q = QDBL ? NDEND : 0;
-    static constexpr int AX = QDBL ? NDEND + 2 * M * PNX : AXR;
-    static constexpr int BYTES = DBYTES + (QDBL ? NDEND + 2 * M * PNX + 4 * NAUX * PNX : NDEND) * 8;
+    static constexpr int TY = ND + (SWIRL ? 2 * NDS : 0);   // swirl: sin^2 of the node rows [patch][NX+1]
+    static constexpr int NDEND = TY + (SWIRL ? NDS : 0);
+    static constexpr int BYTES = DBYTES + NDEND * 8;
 };
 
 // Values a thread carries from one row-iteration to the next.  R is the
@@ -132,18 +125,13 @@ struct PipeState {
     R FYm1[M], FYm2[M], FYp1[M], FYp2[M], FYp3[M];       // y fluxes of the own column, delayed
     double pcur;                                         // swirl: psi at node (c, s+1)
     R smax_x, smax_y;  // largest |s| over the CFL interfaces of each direction
-    bool bad;          // a Riemann problem the reference would stop on (reported as a NaN CFL)
-    int sslot, dslot;  // strip form: slots of the patches this column reads and writes now
 };
 
 // Per-thread constants: column, flags and this thread's element of the rings.
 template <typename R>
 struct PipeThread {
-    double* q;        // q of the patch, offset to column c (strip form: the arena written)
+    double* q;        // q of the patch, offset to column c
     double* qlast;    // qlast of the patch, offset to column c
-    int x, xm, y0;    // strip form: mesh column the values come from, the column itself, first interior row
-    unsigned negx;    // strip form: components negated in this column (solid walls)
-    int mx, ny;       // interior columns and rows (ghost rows included) of the patch or strip
     const double* aux;
     R* rb;            // this thread's element of the R rings
     double* db;       // this thread's element of the FP64 rings
@@ -151,118 +139,55 @@ struct PipeThread {
     const double* ty; // swirl: sin^2 table of the patch's node rows
     double dtdx, dtdy, vty, vtx, tx;
     R rdtdx, rdtdy, rhdtdx, rhdtdy;
-    double* treg;     // time-sync: the patch's conservation registers (nullptr: off)
-    double tdy, tdx;  // time-sync: dt*dy and dt*dx
     int c;
     bool active, save_last, ycol, node;
 };
 
-// The pipelined form accumulates the time-sync registers for the
-// shallow-water Roe solver in FP64, the one whose conservative flux
-// (rpn2_cons_update) the flux store has.
-template <class SOL, bool FUSED>
-__host__ __device__ constexpr bool pipe_time_sync() {
-    return !FUSED && std::is_same_v<SOL, SweRoeT<double, SOL::V5>>;
-}
-
 // ring slot of row s - d when s == J (mod D) is known at compile time
 __host__ __device__ constexpr int cslot(int J, int d, int D) { return ((J - d) % D + D) % D; }
-
-// Row `row` of this thread's column (every component).  Strip form: rows come in
-// order, and the slot is looked up again at patch edges and outside the domain.
-template <class SOL, int NX, bool FUSED>
-__device__ __forceinline__ void load_row(const StepArgs& a, const PipeThread<typename SOL::Real>& T, PipeState<SOL>& S,
-                                         int row, double* v) {
-    constexpr int M = SOL::M;
-    if constexpr (!FUSED) {
-#pragma unroll
-        for (int m = 0; m < M; ++m) v[m] = T.q[((int64_t)m * NX + row) * NX];
-    } else {
-        const StripArgs& g = a.strip;
-        const int ym = T.y0 - 2 + row;
-        bool wall;
-        const int y = strip_inside(ym, g.n, g.bc[2], g.bc[3], wall);
-        if (row == 0 || ym <= 0 || ym >= g.n || (y & ((1 << g.lg) - 1)) == 0) S.sslot = strip_slot(g, T.x, y);
-        const double* p = a.qsrc + ((int64_t)S.sslot * a.q_stride + strip_cell(g, T.x, y));
-        const int plane = g.nxp * g.nxp;
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
-            v[m] = p[m * plane];
-            if constexpr (M > 1)
-                if (((T.negx ^ (wall ? 4u : 0u)) >> m) & 1u) v[m] = -v[m];
-        }
-    }
-}
 
 // One row-iteration.  J >= 0: s == J (mod 4) at compile time, so every ring
 // slot is a constant; STEADY: s in [4, NY-2], where every stage is active for
 // every row and the row-range tests vanish.
-template <class SOL, int NX, int MBC, int AUXK, int NAUX, int PPB, int LIM, int J, bool STEADY, bool FUSED>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int PPB, int LIM, int J, bool STEADY>
 __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                                           const PipeThread<typename SOL::Real>& T, PipeState<SOL>& S, int s) {
     using R = typename SOL::Real;
-    using QT = ring_t<SOL>;
     constexpr int M = SOL::M;
     constexpr int W = SOL::W;
+    constexpr int NX = MX + 2 * MBC;
+    constexpr int NY = NX;
     constexpr bool SWIRL = AUXK == AUX_SWIRL;
-    constexpr bool QDBL = ring_in_fp64<SOL>;
-    // a patch's size is known at compile time, a strip's is not
-    const int MX = FUSED ? T.mx : NX - 2 * MBC, MY = FUSED ? T.ny - 2 * MBC : NX - 2 * MBC;
-    const int NXL = MX + 2 * MBC, NY = MY + 2 * MBC;
-    using L = PipeSmem<NX, PPB, M, W, NAUX, SWIRL, R, QDBL>;
-    QT* qb;  // this thread's element of the state and aux rings
-    if constexpr (QDBL) qb = T.db;
-    else qb = T.rb;
+    using L = PipeSmem<NX, PPB, M, W, NAUX, SWIRL, R>;
+    R* const qb = T.rb;
     const Method<LIM> meth{a};
     // clawpack 5 (clawpack5_flux2.f, clawpack5_step2.f90, clawpack5_step2_wrap.f):
     // fluxes at interfaces 1..mx+1 only, accumulated into cells 1..mx+1, and
     // only the interior cells updated
     constexpr bool V5 = SOL::V5;
-    // f-waves (clawpack46_flux2fw.f): Godunov and correction terms on interfaces
-    // 1..mx+1 only, corrections weighted by sign(s), no transverse part
-    constexpr bool FWAVE = SOL::FWAVE;
-    constexpr bool R15 = V5 || FWAVE;  // fluxes on interfaces MBC..MBC+MX only
-    auto abs_sign = [](R sv) -> R {
-        if constexpr (FWAVE) return copysign(R(1), sv);
-        else return fabs(sv);
-    };
     const int c = T.c;
     auto s2 = [&](int d) -> int { return J >= 0 ? cslot(J, d, 2) : ((s - d) & 1); };
     auto s4 = [&](int d) -> int { return J >= 0 ? cslot(J, d, 4) : ((s - d) & 3); };
     // aux component k of row s-d, column c+dc
-    auto AUXV = [&](int k, int dc, int d) -> QT {
-        if constexpr (NAUX > 0) return k < NAUX ? qb[L::AX + (s4(d) * NAUX + k) * L::PNX + dc] : QT(0);
-        else return QT(0);
+    auto AUXV = [&](int k, int dc, int d) -> R {
+        if constexpr (NAUX > 0) return k < NAUX ? qb[L::AX + (s4(d) * NAUX + k) * L::PNX + dc] : R(0);
+        else return R(0);
     };
 
     // prefetch q(c, s+2); the old value of q(c, s-4) for this iteration's update
     double qnext[M], qold[M];
-    // a fused step writes the interior cells only: the ghost cells it would
-    // update are overwritten by the ghost update that follows every step on a
-    // mesh of one level, and that update is deferred until the ghost cells are read
-    const bool upd = T.active && ((V5 || FUSED) ? (s - 4 >= MBC && s - 4 <= MBC + MY - 1 && c >= MBC && c <= MBC + MX - 1)
-                                                : ((STEADY || (s - 4 >= 0 && s - 4 <= NY - 2)) && c <= NX - 2));
-    int64_t dst = 0;  // strip form: where cell (c, s-4) lives in the arenas
-    if constexpr (FUSED) {
-        if (upd) {
-            const int y = T.y0 + s - 4 - MBC;
-            if (s - 4 == MBC || (y & ((1 << a.strip.lg) - 1)) == 0) S.dslot = strip_slot(a.strip, T.x, y);
-            dst = (int64_t)S.dslot * a.q_stride + strip_cell(a.strip, T.x, y);
-        }
-    }
+    const bool upd = T.active && (V5 ? (s - 4 >= MBC && s - 4 <= MBC + MX - 1 && c >= MBC && c <= MBC + MX - 1)
+                                     : ((STEADY || (s - 4 >= 0 && s - 4 <= NY - 2)) && c <= NX - 2));
     {
-        // prefetch two rows ahead; the last steady iteration of a patch
-        // (s = 4 + 4*((NY-5)/4) - 1) still has row s+2 inside it for the sizes built here
-        constexpr bool STEADY_IN = !FUSED && 4 + 4 * ((NX - 5) / 4) + 1 < NX;
+        // prefetch two rows ahead; the last steady iteration (s = 4 + 4*((NY-5)/4) - 1)
+        // still has row s+2 inside the patch for the patch sizes built here
+        constexpr bool STEADY_IN = 4 + 4 * ((NY - 5) / 4) + 1 < NY;
         const bool on = T.active && ((STEADY && STEADY_IN) || s + 2 < NY);
 #pragma unroll
-        for (int m = 0; m < M; ++m) qnext[m] = 0.0;
-        if (on) load_row<SOL, NX, FUSED>(a, T, S, s + 2, qnext);
-#pragma unroll
         for (int m = 0; m < M; ++m) {
+            qnext[m] = on ? T.q[((int64_t)m * NY + s + 2) * NX] : 0.0;
             if constexpr (PipeState<SOL>::DELAY) qold[m] = S.q_m4[m];
-            else if constexpr (FUSED) qold[m] = upd ? a.qsrc[dst + m * a.strip.nxp * a.strip.nxp] : 0.0;
-            else qold[m] = upd ? T.q[((int64_t)m * NX + s - 4) * NX] : 0.0;
+            else qold[m] = upd ? T.q[((int64_t)m * NY + s - 4) * NX] : 0.0;
         }
     }
 
@@ -276,7 +201,7 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
         for (int m = 0; m < M; ++m) {
             double gxd = 0.0, gxu = 0.0;
             if (xint) {
-                if (c + 1 <= NXL - 1) {
+                if (c + 1 <= NX - 1) {
                     gxd = -(double)gl[(0 * M + m) * L::PNX + 1] - (double)S.gRmx[m];
                     gxu = -(double)gl[(1 * M + m) * L::PNX + 1] - (double)S.gRpx[m];
                 } else {
@@ -292,27 +217,11 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
     // ---------------- S5: update cell row r = s-4 ----------------
     {
         const int r = s - 4;
-        // time-sync: the boundary fluctuations of the cells next to the patch
-        // edges, inside and outside (clawpack46_time_sync_accumulate_waves,
-        // clawpack5_time_sync_accumulate_waves), which the clawpack 5 update
-        // computes but does not apply to the ghost cells
-        constexpr bool TSYNC = pipe_time_sync<SOL, FUSED>();
-        const int i = c - MBC + 1, j = r - MBC + 1;
-        bool tsr = false;
-        if constexpr (TSYNC) {
-            const bool iin = i >= 1 && i <= MX, jin = j >= 1 && j <= MX;
-            const bool iedge = i == 0 || i == 1 || i == MX || i == MX + 1;
-            const bool jedge = j == 0 || j == 1 || j == MX || j == MX + 1;
-            tsr = T.treg != nullptr && T.active && ((iedge && jin) || (jedge && iin));
-        }
-        if (upd || tsr) {
+        if (upd) {
             const R* fx = T.rb + L::FX + s4(4) * (2 * M * L::PNX);
             const double* gy = T.db + L::GY + s4(4) * (2 * M * L::PNX);
 #pragma unroll
             for (int m = 0; m < M; ++m) {
-                double* qp;
-                if constexpr (FUSED) qp = T.q + dst + m * a.strip.nxp * a.strip.nxp;
-                else qp = T.q + ((int64_t)m * NX + r) * NX;
                 const double fxm1 = fx[(0 * M + m) * L::PNX + 1];  // FP32 flux parts widen exactly
                 const double fxp0 = fx[(1 * M + m) * L::PNX];
                 const double gyu_l = (c >= 1) ? gy[(1 * M + m) * L::PNX - 1] : 0.0;
@@ -323,28 +232,7 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 const double fpv = (fxp0 + gyu_l) + gyd;   // fp(i, j)
                 const double gmv = GXs_new[m] + (double)S.FYm2[m];    // gm(i, j+1)
                 const double gpv = S.GXs_prev[m] + (double)S.FYp3[m];  // gp(i, j)
-                if (upd) *qp = qold[m] - T.dtdx * (fmv - fpv) - T.dtdy * (gmv - gpv);
-                if constexpr (TSYNC) {
-                    if (tsr) {
-                        // each register element has exactly one writer
-                        const RegLayout RL{MX, MX, M};
-                        double* Rg = T.treg;
-                        if (j >= 1 && j <= MX) {
-                            const int k = (j - 1) + MX * m;
-                            if (i == 1) Rg[RL.fp(0) + k] = Rg[RL.fp(0) + k] - T.tdy * fpv;
-                            if (i == 0) Rg[RL.fm(0) + k] = Rg[RL.fm(0) + k] + T.tdy * fmv;       // fm(1, j)
-                            if (i == MX) Rg[RL.fm(1) + k] = Rg[RL.fm(1) + k] + T.tdy * fmv;      // fm(mx+1, j)
-                            if (i == MX + 1) Rg[RL.fp(1) + k] = Rg[RL.fp(1) + k] - T.tdy * fpv;  // fp(mx+1, j)
-                        }
-                        if (i >= 1 && i <= MX) {
-                            const int k = (i - 1) + MX * m;
-                            if (j == 1) Rg[RL.gp(0) + k] = Rg[RL.gp(0) + k] - T.tdx * gpv;
-                            if (j == 0) Rg[RL.gm(0) + k] = Rg[RL.gm(0) + k] + T.tdx * gmv;       // gm(i, 1)
-                            if (j == MX) Rg[RL.gm(1) + k] = Rg[RL.gm(1) + k] + T.tdx * gmv;      // gm(i, my+1)
-                            if (j == MX + 1) Rg[RL.gp(1) + k] = Rg[RL.gp(1) + k] - T.tdx * gpv;  // gp(i, my+1)
-                        }
-                    }
-                }
+                T.q[((int64_t)m * NY + r) * NX] = qold[m] - T.dtdx * (fmv - fpv) - T.dtdy * (gmv - gpv);
             }
         }
 #pragma unroll
@@ -356,7 +244,7 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
         const int k = s - 2;
         if (T.active && (STEADY || (k >= 0 && k <= NY - 2))) {
             R* fx = T.rb + L::FX + s4(2) * (2 * M * L::PNX);
-            const bool xint = (STEADY || k >= 1) && (R15 ? (c >= MBC && c <= MBC + MX) : c >= 1);
+            const bool xint = (STEADY || k >= 1) && (V5 ? (c >= MBC && c <= MBC + MX) : c >= 1);
             if (xint) {
                 const R* xw = T.rb + L::XW + s2(2) * (W * M * L::PNX);
                 R cq[M];
@@ -390,12 +278,12 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                         R acc;
                         {
                             const R as = fabs(S.xsl[0]);
-                            acc = abs_sign(S.xsl[0]) * (R(1) - as * T.rdtdx) * S.xwl[0][m];
+                            acc = as * (R(1) - as * T.rdtdx) * S.xwl[0][m];
                         }
 #pragma unroll
                         for (int mw = 1; mw < W; ++mw) {
                             const R as = fabs(S.xsl[mw]);
-                            acc = acc + abs_sign(S.xsl[mw]) * (R(1) - as * T.rdtdx) * S.xwl[mw][m];
+                            acc = acc + as * (R(1) - as * T.rdtdx) * S.xwl[mw][m];
                         }
                         cq[m] = acc;
                     }
@@ -403,14 +291,14 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 R am[M], ap[M];
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
-                    R fmv = (c <= NXL - 2) ? S.xam[m] : R(0);
+                    R fmv = (c <= NX - 2) ? S.xam[m] : R(0);
                     R fpv = (c <= NX - 2) ? -S.xap[m] : R(0);
                     if (meth.second_order()) { fmv = fmv + R(0.5) * cq[m]; fpv = fpv + R(0.5) * cq[m]; }
                     fx[(0 * M + m) * L::PNX] = fmv;
                     fx[(1 * M + m) * L::PNX] = fpv;
                     am[m] = S.xam[m];
                     ap[m] = S.xap[m];
-                    if (meth.transverse2() && c <= NXL - 2) { am[m] = am[m] + cq[m]; ap[m] = ap[m] - cq[m]; }
+                    if (meth.transverse2() && c <= NX - 2) { am[m] = am[m] + cq[m]; ap[m] = ap[m] - cq[m]; }
                 }
                 R* gl = T.rb + L::GL + s2(2) * (2 * M * L::PNX);
                 if (meth.transverse()) {
@@ -441,7 +329,7 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 for (int m = 0; m < M; ++m) {
                     fx[(0 * M + m) * L::PNX] = R(0);
                     fx[(1 * M + m) * L::PNX] = R(0);
-                    if constexpr (R15) {  // read by the cell to the left (mx+1 at the right end)
+                    if constexpr (V5) {  // read by the cell to the left (mx+1 at the right end)
                         R* gl = T.rb + L::GL + s2(2) * (2 * M * L::PNX);
                         gl[(0 * M + m) * L::PNX] = R(0);
                         gl[(1 * M + m) * L::PNX] = R(0);
@@ -455,20 +343,14 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
     {
         const int k = s - 1;
         if (T.active && (STEADY || (k >= 1 && k <= NY - 2)) && c >= 1) {
-            const QT* qr = qb + L::Q + s2(1) * (M * L::PNX);
-            QT qL[M], qR[M];
+            const R* qr = qb + L::Q + s2(1) * (M * L::PNX);
+            R qL[M], qR[M];
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 qL[m] = qr[m * L::PNX - 1];
-                qR[m] = QT(S.q_m1[m]);
+                qR[m] = R(S.q_m1[m]);
             }
-            if constexpr (FWAVE) {
-                bool bad = false;
-                sol.rpn2b(1, qL, qR, AUXV(0, -1, 1), AUXV(0, 0, 1), S.xwl, S.xsl, S.xam, S.xap, bad);
-                S.bad = S.bad || bad;
-            } else {
-                sol.rpn2(1, qL, qR, AUXV(0, 0, 1), S.xwl, S.xsl, S.xam, S.xap, S.xR);
-            }
+            sol.rpn2(1, qL, qR, AUXV(0, 0, 1), S.xwl, S.xsl, S.xam, S.xap, S.xR);
             R* xw = T.rb + L::XW + s2(1) * (W * M * L::PNX);
 #pragma unroll
             for (int mw = 0; mw < W; ++mw) {
@@ -492,27 +374,21 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
 #pragma unroll
         for (int m = 0; m < M; ++m) yam_n[m] = yap_n[m] = R(0);
         if (T.active && (STEADY || s < NY)) {
-            QT* qr = qb + L::Q + s2(0) * (M * L::PNX);
+            R* qr = qb + L::Q + s2(0) * (M * L::PNX);
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 if (T.save_last) T.qlast[((int64_t)m * NX + s) * NX] = S.qcur[m];
-                qr[m * L::PNX] = QT(S.qcur[m]);
+                qr[m * L::PNX] = R(S.qcur[m]);
             }
             // raw y-interface s (between rows s-1 and s)
             if (T.ycol && (STEADY || s >= 1)) {
-                QT qD[M], qU[M];
+                R qD[M], qU[M];
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
-                    qD[m] = QT(S.q_m1[m]);
-                    qU[m] = QT(S.qcur[m]);
+                    qD[m] = R(S.q_m1[m]);
+                    qU[m] = R(S.qcur[m]);
                 }
-                if constexpr (FWAVE) {
-                    bool bad = false;
-                    sol.rpn2b(2, qD, qU, AUXV(0, 0, 1), AUXV(0, 0, 0), yw_n, ys_n, yam_n, yap_n, bad);
-                    S.bad = S.bad || bad;
-                } else {
-                    sol.rpn2(2, qD, qU, AUXV(1, 0, 0), yw_n, ys_n, yam_n, yap_n, yR_n);
-                }
+                sol.rpn2(2, qD, qU, AUXV(1, 0, 0), yw_n, ys_n, yam_n, yap_n, yR_n);
 #pragma unroll
                 for (int mw = 0; mw < W; ++mw) {
                     R d = S.yw_f[mw][0] * yw_n[mw][0];
@@ -534,11 +410,11 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
         }
         // clawpack 5: interfaces MBC..MBC+MX carry fluxes; f = MBC+MX+1 only
         // closes the transverse sum of cell row MBC+MX
-        const bool yblk = T.ycol && (R15 ? (f >= MBC && f <= MBC + MY + 1) : (STEADY || (f >= 1 && f <= NY - 1)));
+        const bool yblk = T.ycol && (V5 ? (f >= MBC && f <= MBC + MX + 1) : (STEADY || (f >= 1 && f <= NY - 1)));
         if (yblk) {
-            const bool fact = !R15 || f <= MBC + MY;
-            const bool inner = R15 ? fact : (STEADY || (f >= MBC && f <= MBC + MY));
-            const bool god = R15 ? fact : (STEADY || f <= NY - 2);
+            const bool fact = !V5 || f <= MBC + MX;
+            const bool inner = V5 ? fact : (STEADY || (f >= MBC && f <= MBC + MX));
+            const bool god = V5 ? fact : (STEADY || f <= NY - 2);
             R w[W][M];
 #pragma unroll
             for (int mw = 0; mw < W; ++mw)
@@ -572,12 +448,12 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                     R acc;
                     {
                         const R as = fabs(S.ys_f[0]);
-                        acc = abs_sign(S.ys_f[0]) * (R(1) - as * T.rdtdy) * w[0][m];
+                        acc = as * (R(1) - as * T.rdtdy) * w[0][m];
                     }
 #pragma unroll
                     for (int mw = 1; mw < W; ++mw) {
                         const R as = fabs(S.ys_f[mw]);
-                        acc = acc + abs_sign(S.ys_f[mw]) * (R(1) - as * T.rdtdy) * w[mw][m];
+                        acc = acc + as * (R(1) - as * T.rdtdy) * w[mw][m];
                     }
                     cq[m] = acc;
                 }
@@ -609,7 +485,7 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 for (int m = 0; m < M; ++m) gLm[m] = gLp[m] = gRm[m] = gRp[m] = R(0);
             }
             // cell row f-1 is complete: gadd(f-1,.,1) = (0 - gL(f)) - gR(f-1)
-            if (R15 ? (f - 1 >= MBC && f - 1 <= MBC + MY) : (STEADY || f - 1 >= 1)) {
+            if (V5 ? (f - 1 >= MBC && f - 1 <= MBC + MX) : (STEADY || f - 1 >= 1)) {
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
                     GYd[m] = -(double)gLm[m] - (double)S.gRm_prev[m];
@@ -667,19 +543,16 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 const double pn = psi_node<R>(T.tx, T.ty[s + 2]);
                 if (T.node) T.nb[s2(-2) * L::NDS] = pn;
                 if (T.active) {
-                    QT* ax = qb + L::AX + s4(-1) * (NAUX * L::PNX);
-                    ax[0 * L::PNX] = QT(T.vty * (pn - S.pcur));
-                    ax[1 * L::PNX] = QT(-T.vtx * (T.nb[s2(-1) * L::NDS + 1] - S.pcur));
+                    R* ax = qb + L::AX + s4(-1) * (NAUX * L::PNX);
+                    ax[0 * L::PNX] = R(T.vty * (pn - S.pcur));
+                    ax[1 * L::PNX] = R(-T.vtx * (T.nb[s2(-1) * L::NDS + 1] - S.pcur));
                 }
                 S.pcur = pn;
             } else if constexpr (AUXK == AUX_STORED) {
                 if (T.active) {
-                    QT* ax = qb + L::AX + s4(-1) * (NAUX * L::PNX);
+                    R* ax = qb + L::AX + s4(-1) * (NAUX * L::PNX);
 #pragma unroll
-                    for (int kk = 0; kk < NAUX; ++kk) {
-                        if constexpr (FUSED) ax[kk * L::PNX] = QT(strip_aux(a, T.xm, T.y0 - 2 + s + 1, kk));
-                        else ax[kk * L::PNX] = QT(T.aux[(kk * NX + s + 1) * NX]);
-                    }
+                    for (int kk = 0; kk < NAUX; ++kk) ax[kk * L::PNX] = R(T.aux[(kk * NY + s + 1) * NX]);
                 }
             }
         }
@@ -703,17 +576,17 @@ constexpr bool pipe_six_ctas() {
     return sizeof(typename SOL::Real) == 4 && SOL::M == 1;
 }
 
-// NX: columns of a patch, ghost columns included; of a strip (FUSED): the most it has.
-template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
 __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     constexpr int M = SOL::M;
     constexpr int W = SOL::W;
+    constexpr int NX = MX + 2 * MBC;
+    constexpr int NY = NX;
     constexpr bool SWIRL = AUXK == AUX_SWIRL;
     constexpr int TPP = pipe_threads_per_patch<NX, SWIRL>();
     constexpr int PPB = TPB / TPP;
     using R = typename SOL::Real;
-    using QT = ring_t<SOL>;
-    using L = PipeSmem<NX, PPB, M, W, NAUX, SWIRL, R, ring_in_fp64<SOL>>;
+    using L = PipeSmem<NX, PPB, M, W, NAUX, SWIRL, R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* const rsm = reinterpret_cast<R*>(smem_raw);
     double* const dsm = reinterpret_cast<double*>(smem_raw + L::DBYTES);
@@ -725,58 +598,25 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     const int pl = t / TPP;
     const int c = t - pl * TPP;
     const int pg = blockIdx.x * PPB + pl;
-    // a strip: interior columns [x0, x0 + mxs) and rows [y0, y0 + mys) of the mesh
-    const int sx = FUSED ? blockIdx.x % a.strip.nsx : 0, sy = FUSED ? blockIdx.x / a.strip.nsx : 0;
-    const int x0 = sx * a.strip.w, y0 = sy * a.strip.h;
-    const int mxs = FUSED ? min(a.strip.w, a.strip.n - x0) : NX - 2 * MBC;
-    const int mys = FUSED ? min(a.strip.h, a.strip.n - y0) : NX - 2 * MBC;
-    const int NY = FUSED ? mys + 2 * MBC : NX;
-    const bool patch_ok = FUSED ? pl == 0 && c <= mxs + 2 * MBC : (pl < PPB) && (pg < a.npatches);
-    const bool active = patch_ok && c < mxs + 2 * MBC;
+    const bool patch_ok = (pl < PPB) && (pg < a.npatches);
+    const bool active = patch_ok && c < NX;
     const int pls = patch_ok ? pl : 0;  // threads without a patch read (never write) patch 0's rows
     const int cc = c < NX ? c : NX - 1;
     const PatchDesc* D = (a.desc && patch_ok) ? a.desc + pg : nullptr;  // mixed-solve launch
-    int slot = 0;
-    if constexpr (FUSED) slot = __ldg(a.strip.grid);  // every patch has the same cell size
-    else slot = (patch_ok && !a.desc) ? a.slots[pg] : 0;
-    PatchMeta meta = D ? D->meta : (FUSED || patch_ok ? a.meta[slot] : PatchMeta{0, 0, 1, 1, 0, 0});
-    if constexpr (FUSED) {
-        // the strip's own corner: the mesh's cell edges are exact multiples of its spacing
-        meta.xlower = a.strip.ax + (double)x0 * meta.dx;
-        meta.ylower = a.strip.ay + (double)y0 * meta.dy;
-    }
+    const int slot = (patch_ok && !a.desc) ? a.slots[pg] : 0;
+    const PatchMeta meta = D ? D->meta : (patch_ok ? a.meta[slot] : PatchMeta{0, 0, 1, 1, 0, 0});
     const int req = D ? D->req : -1;
     SOL sol{R(a.grav), R(a.gamma), R(a.gamma1), R(a.drytol)};
-    if constexpr (SOL::FWAVE) {
-        sol.gdbl = a.grav;
-        sol.drytol_d = a.drytol;
-        sol.ctol2 = sqrt(dmax(a.drytol * a.grav, 1e-6));
-    }
 
     PipeThread<R> T;
     T.c = cc;
     T.active = active;
     T.node = SWIRL && patch_ok;
     T.save_last = active && (meta.flags & PATCH_SAVE_LAST);
-    T.ycol = active && c >= 1 && c <= mxs + 2 * MBC - 2;
-    T.mx = mxs;
-    T.ny = NY;
-    if constexpr (FUSED) T.q = a.q;
-    else T.q = (D ? D->q : a.q + (int64_t)slot * a.q_stride) + cc;
+    T.ycol = active && c >= 1 && c <= NX - 2;
+    T.q = (D ? D->q : a.q + (int64_t)slot * a.q_stride) + cc;
     T.qlast = (D ? D->qlast : a.qlast + (int64_t)slot * a.q_stride) + cc;
-    T.x = T.xm = T.y0 = 0;
-    T.negx = 0u;
-    PipeState<SOL> S;
-    S.sslot = S.dslot = 0;
-    if constexpr (FUSED) {
-        T.save_last = false;  // a mesh of one level has no patch with finer neighbours
-        bool wall;
-        T.xm = x0 - MBC + c;
-        T.x = strip_inside(T.xm, a.strip.n, a.strip.bc[0], a.strip.bc[1], wall);
-        T.negx = wall ? 2u : 0u;
-        T.y0 = y0;
-    }
-    T.aux = (AUXK == AUX_STORED && active && !FUSED) ? (D ? D->aux : a.aux + (int64_t)slot * a.aux_stride) + cc : nullptr;
+    T.aux = (AUXK == AUX_STORED && active) ? (D ? D->aux : a.aux + (int64_t)slot * a.aux_stride) + cc : nullptr;
     T.rb = rsm + pls * NX + cc;
     T.db = dsm + pls * NX + cc;
     T.nb = dsm + L::ND + pls * (NX + 1) + c;
@@ -792,24 +632,12 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     T.vty = vt / meta.dy;
     T.vtx = vt / meta.dx;
     T.tx = 0.0;
-    T.treg = nullptr;
-    T.tdy = T.tdx = 0.0;
-    if constexpr (pipe_time_sync<SOL, FUSED>()) {
-        if (a.treg && patch_ok && !D) {
-            T.treg = a.treg + (int64_t)slot * a.treg_stride;
-            T.tdy = dt * meta.dy;
-            T.tdx = dt * meta.dx;
-        }
-    }
 
-#pragma unroll
-    for (int m = 0; m < M; ++m) S.qcur[m] = S.qpre[m] = 0.0;
-    if (active) {
-        load_row<SOL, NX, FUSED>(a, T, S, 0, S.qcur);
-        load_row<SOL, NX, FUSED>(a, T, S, 1, S.qpre);
-    }
+    PipeState<SOL> S;
 #pragma unroll
     for (int m = 0; m < M; ++m) {
+        S.qcur[m] = active ? T.q[(int64_t)m * NY * NX] : 0.0;
+        S.qpre[m] = active ? T.q[((int64_t)m * NY + 1) * NX] : 0.0;
         S.q_m1[m] = 0.0;
         S.q_m2[m] = S.q_m3[m] = S.q_m4[m] = 0.0;
         S.yam_f[m] = S.yap_f[m] = R(0);
@@ -829,7 +657,6 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     S.xR = typename SOL::Roe{};
     S.pcur = 0.0;
     S.smax_x = S.smax_y = R(0);
-    S.bad = false;
 
     // ---- prologue: aux row 0 ----
     if constexpr (SWIRL) {
@@ -845,14 +672,7 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
             const double y = meta.ylower + (double)(c - MBC) * meta.dy;
             const double sx = sin(pi * x), sy = sin(pi * y);
             T.tx = sx * sx;
-            if constexpr (FUSED) {
-                for (int k = t; k <= NY; k += TPB) {
-                    const double sk = sin(pi * (meta.ylower + (double)(k - MBC) * meta.dy));
-                    dsm[L::TY + k] = sk * sk;
-                }
-            } else {
-                if (T.node) dsm[L::TY + pls * (NX + 1) + c] = sy * sy;
-            }
+            if (T.node) dsm[L::TY + pls * (NX + 1) + c] = sy * sy;
         }
         __syncthreads();
         const double p0 = psi_node<R>(T.tx, T.ty[0]), p1 = psi_node<R>(T.tx, T.ty[1]);
@@ -862,42 +682,35 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
         }
         __syncthreads();
         if (active) {
-            T.rb[L::AX + 0 * L::PNX] = QT(T.vty * (p1 - p0));
-            T.rb[L::AX + 1 * L::PNX] = QT(-T.vtx * (T.nb[1] - p0));
+            T.rb[L::AX + 0 * L::PNX] = R(T.vty * (p1 - p0));
+            T.rb[L::AX + 1 * L::PNX] = R(-T.vtx * (T.nb[1] - p0));
         }
         S.pcur = p1;
     } else if constexpr (AUXK == AUX_STORED) {
         if (active) {
 #pragma unroll
-            for (int k = 0; k < NAUX; ++k) {
-                double v;
-                if constexpr (FUSED) v = strip_aux(a, T.xm, T.y0 - 2, k);
-                else v = T.aux[k * NX * NX];
-                if constexpr (ring_in_fp64<SOL>) T.db[L::AX + k * L::PNX] = v;
-                else T.rb[L::AX + k * L::PNX] = QT(v);
-            }
+            for (int k = 0; k < NAUX; ++k) T.rb[L::AX + k * L::PNX] = R(T.aux[k * NY * NX]);
         }
     }
     __syncthreads();
 
     // ---- rows: ramp-up, steady state (unrolled by the ring period 4), ramp-down ----
     int s = 0;
-    for (; s < 4; ++s) pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, -1, false, FUSED>(a, sol, T, S, s);
-    const int NSTEADY = NY - 5;  // s = 4 .. NY-2
+    for (; s < 4; ++s) pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, -1, false>(a, sol, T, S, s);
+    constexpr int NSTEADY = NY - 5;  // s = 4 .. NY-2
     for (int rnd = 0; rnd < NSTEADY / 4; ++rnd, s += 4) {
-        pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, 0, true, FUSED>(a, sol, T, S, s);
-        pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, 1, true, FUSED>(a, sol, T, S, s + 1);
-        pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, 2, true, FUSED>(a, sol, T, S, s + 2);
-        pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, 3, true, FUSED>(a, sol, T, S, s + 3);
+        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 0, true>(a, sol, T, S, s);
+        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 1, true>(a, sol, T, S, s + 1);
+        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 2, true>(a, sol, T, S, s + 2);
+        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 3, true>(a, sol, T, S, s + 3);
     }
-    for (; s <= NY + 2; ++s) pipe_iter<SOL, NX, MBC, AUXK, NAUX, PPB, LIM, -1, false, FUSED>(a, sol, T, S, s);
+    for (; s <= NY + 2; ++s) pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, -1, false>(a, sol, T, S, s);
 
     // ---- CFL: warp max, one atomic per warp ----
     // flux2: cfl = max(cfl, dtdx*s, -dtdx*s) over the interfaces.  Rounding is
     // monotone, so max_i fl(dtdx*|s_i|) == fl(dtdx * max_i |s_i|): one product
     // per direction gives the reference's value exactly.
     double cfl = (double)nanmax(T.rdtdx * S.smax_x, T.rdtdy * S.smax_y);
-    if (S.bad) cfl = __longlong_as_double(0x7ff8000000000000LL);  // NaN: wins the max, reported by the host
     if (a.desc) {
         // patches of different solves share warps: reduce over the lanes of each
         // solve (max of the non-negative bit patterns, high word then low word)
@@ -914,21 +727,21 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     }
 }
 
-template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
 __global__ void __launch_bounds__(TPB) step_kernel_pipe(const StepArgs a) {
-    step_pipe_body<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>(a);
+    step_pipe_body<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(a);
 }
 
-template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
 __global__ void __launch_bounds__(TPB, 6) step_kernel_pipe_six(const StepArgs a) {
-    step_pipe_body<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>(a);
+    step_pipe_body<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(a);
 }
 
 // the one kernel of the two that a form uses (only that one is instantiated)
-template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
 constexpr auto pipe_kernel() {
-    if constexpr (pipe_six_ctas<SOL>()) return step_kernel_pipe_six<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>;
-    else return step_kernel_pipe<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>;
+    if constexpr (pipe_six_ctas<SOL>()) return step_kernel_pipe_six<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>;
+    else return step_kernel_pipe<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>;
 }
 
 // ---------------------------------------------------------------------------
@@ -936,45 +749,24 @@ constexpr auto pipe_kernel() {
 // ---------------------------------------------------------------------------
 namespace {
 
-template <class SOL, int NX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
 cudaError_t launch_pipe_one(const StepArgs& a, cudaStream_t st) {
+    constexpr int NX = MX + 2 * MBC;
     constexpr int PPB = TPB / pipe_threads_per_patch<NX, AUXK == AUX_SWIRL>();
     static_assert(PPB >= 1, "patch wider than the CTA");
-    using L = PipeSmem<NX, PPB, SOL::M, SOL::W, NAUX, AUXK == AUX_SWIRL, typename SOL::Real, ring_in_fp64<SOL>>;
-    constexpr auto kernel = pipe_kernel<SOL, NX, MBC, AUXK, NAUX, TPB, LIM, FUSED>();
-    if constexpr (!FUSED) {
-        const size_t bytes = (size_t)L::BYTES;
-        static bool configured = false;
-        if (!configured) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-            if (e != cudaSuccess) return e;
-            configured = true;
-        }
-        const int blocks = (a.npatches + PPB - 1) / PPB;
-        if (blocks == 0) return cudaSuccess;
-        kernel<<<blocks, TPB, bytes, st>>>(a);
-        return cudaGetLastError();
-    } else {
-        // bytes of a strip of h rows: its table of node rows replaces the patches'
-        constexpr bool SWIRL = AUXK == AUX_SWIRL;
-        auto bytes_of = [](int h) { return (int)(L::BYTES + (SWIRL ? (h + 2 * MBC + 1 - L::NDS) * 8 : 0)); };
-        static std::atomic<int> per_wave{0};
-        if (per_wave.load() == 0) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 bytes_of(kStripRowsMax));
-            if (e != cudaSuccess) return e;
-            int dev = 0, sms = 0, occ = 0;
-            if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-            if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, TPB, bytes_of(256))) != cudaSuccess)
-                return e;
-            per_wave.store(std::max(1, sms * occ));
-        }
-        StepArgs b = a;
-        strip_plan(b.strip, NX - 2 * MBC, per_wave.load());
-        kernel<<<b.strip.nsx * b.strip.nsy, TPB, bytes_of(b.strip.h), st>>>(b);
-        return cudaGetLastError();
+    using L = PipeSmem<NX, PPB, SOL::M, SOL::W, NAUX, AUXK == AUX_SWIRL, typename SOL::Real>;
+    const size_t bytes = (size_t)L::BYTES;
+    constexpr auto kernel = pipe_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>();
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return e;
+        configured = true;
     }
+    const int blocks = (a.npatches + PPB - 1) / PPB;
+    if (blocks == 0) return cudaSuccess;
+    kernel<<<blocks, TPB, bytes, st>>>(a);
+    return cudaGetLastError();
 }
 
 // Limiter specialisation: every wave limited with the same code and order (2, 2).
@@ -987,29 +779,23 @@ int fixed_limiter(const StepArgs& a) {
     return (l == 3 || l == 4) ? l : 0;
 }
 
-template <class SOL, int NX, int AUXK, int NAUX, bool FUSED>
+template <class SOL, int MX, int AUXK, int NAUX>
 cudaError_t launch_pipe_lim(const StepArgs& a, cudaStream_t st) {
     switch (fixed_limiter<SOL>(a)) {
-        case 3: return launch_pipe_one<SOL, NX, 2, AUXK, NAUX, 128, 3, FUSED>(a, st);
-        case 4: return launch_pipe_one<SOL, NX, 2, AUXK, NAUX, 128, 4, FUSED>(a, st);
-        default: return launch_pipe_one<SOL, NX, 2, AUXK, NAUX, 128, 0, FUSED>(a, st);
+        case 3: return launch_pipe_one<SOL, MX, 2, AUXK, NAUX, 128, 3>(a, st);
+        case 4: return launch_pipe_one<SOL, MX, 2, AUXK, NAUX, 128, 4>(a, st);
+        default: return launch_pipe_one<SOL, MX, 2, AUXK, NAUX, 128, 0>(a, st);
     }
 }
 
-template <class SOL, int AUXK, int NAUX, bool FUSED>
+template <class SOL, int AUXK, int NAUX>
 cudaError_t launch_pipe_mx(int mx, int mbc, const StepArgs& a, cudaStream_t st) {
     if (mbc != 2) return cudaErrorNotSupported;
-    if constexpr (FUSED) {
-        // strips take patches of any size; with the swirl velocities the last
-        // thread of the CTA works on a node column alone
-        return launch_pipe_lim<SOL, AUXK == AUX_SWIRL ? 127 : 128, AUXK, NAUX, true>(a, st);
-    } else {
-        switch (mx) {
-            case 8: return launch_pipe_lim<SOL, 12, AUXK, NAUX, false>(a, st);
-            case 16: return launch_pipe_lim<SOL, 20, AUXK, NAUX, false>(a, st);
-            case 32: return launch_pipe_lim<SOL, 36, AUXK, NAUX, false>(a, st);
-            default: return cudaErrorNotSupported;
-        }
+    switch (mx) {
+        case 8: return launch_pipe_lim<SOL, 8, AUXK, NAUX>(a, st);
+        case 16: return launch_pipe_lim<SOL, 16, AUXK, NAUX>(a, st);
+        case 32: return launch_pipe_lim<SOL, 32, AUXK, NAUX>(a, st);
+        default: return cudaErrorNotSupported;
     }
 }
 
@@ -1018,16 +804,20 @@ cudaError_t launch_pipe_mx(int mx, int mbc, const StepArgs& a, cudaStream_t st) 
 // cudaErrorNotSupported: no pipelined form for this (solver, mx, mbc, aux).
 // R: compute type of the Riemann solves, limiters and transverse parts;
 // V5: the clawpack 5 update (fc2d_clawpack5) instead of clawpack 4.6.
-template <typename R, bool V5, bool FUSED>
+template <typename R, bool V5>
 cudaError_t launch_step_pipe_v(int solver, int aux_kind, int mwaves, int mx, int my, int mbc, const StepArgs& a,
                                cudaStream_t st) {
     if (mx != my) return cudaErrorNotSupported;
     switch (solver) {
         case SOLVER_ADVECTION:
             if (mwaves != 1) return cudaErrorNotSupported;
-            if (aux_kind == AUX_SWIRL) return launch_pipe_mx<AdvectionSolver<1, R, V5>, AUX_SWIRL, 2, FUSED>(mx, mbc, a, st);
+            if (a.strip.grid) {
+                if constexpr (std::is_same_v<R, float>) return launch_step_adv_mixed(aux_kind, V5 ? 5 : 4, a, st);
+                else return launch_step_adv(aux_kind, V5 ? 5 : 4, a, st);
+            }
+            if (aux_kind == AUX_SWIRL) return launch_pipe_mx<AdvectionSolver<1, R, V5>, AUX_SWIRL, 2>(mx, mbc, a, st);
             if (aux_kind == AUX_STORED && a.maux >= 2)
-                return launch_pipe_mx<AdvectionSolver<1, R, V5>, AUX_STORED, 2, FUSED>(mx, mbc, a, st);
+                return launch_pipe_mx<AdvectionSolver<1, R, V5>, AUX_STORED, 2>(mx, mbc, a, st);
             return cudaErrorNotSupported;
         case SOLVER_SWE_ROE:
             if (mwaves != 3 || aux_kind != AUX_NONE) return cudaErrorNotSupported;
@@ -1048,13 +838,14 @@ cudaError_t launch_step_pipe_v(int solver, int aux_kind, int mwaves, int mx, int
     else return launch_split_geoclaw(mx, a, st);
 }
 
-// FUSED: the ghost-exchange-fused form (a.strip and a.qsrc set; mesh of one level)
-template <typename R, bool FUSED>
+// With a.strip set (a.qsrc another arena than a.q) the ghost-exchange-fused form of a
+// mesh of one level.
+template <typename R>
 cudaError_t launch_step_pipe_t(int solver, int aux_kind, int mwaves, int mx, int my, int mbc, int claw_version,
                                const StepArgs& a, cudaStream_t st) {
-    if (FUSED != (a.strip.grid != nullptr) || (FUSED && (a.desc || !a.qsrc || a.qsrc == a.q))) return cudaErrorInvalidValue;
-    if (claw_version == 5) return launch_step_pipe_v<R, true, FUSED>(solver, aux_kind, mwaves, mx, my, mbc, a, st);
-    return launch_step_pipe_v<R, false, FUSED>(solver, aux_kind, mwaves, mx, my, mbc, a, st);
+    if (a.strip.grid && (a.desc || !a.qsrc || a.qsrc == a.q)) return cudaErrorInvalidValue;
+    if (claw_version == 5) return launch_step_pipe_v<R, true>(solver, aux_kind, mwaves, mx, my, mbc, a, st);
+    return launch_step_pipe_v<R, false>(solver, aux_kind, mwaves, mx, my, mbc, a, st);
 }
 
 }  // namespace fcb

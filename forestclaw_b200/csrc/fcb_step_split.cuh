@@ -892,7 +892,7 @@ cudaError_t launch_split_one(const StepArgs& a, cudaStream_t st) {
     StepArgs b = a;
     int blocks;
     if constexpr (MXP == 0) {
-        strip_plan(b.strip, HALF - 4, per_wave.load());
+        strip_plan(b.strip, HALF - 4, per_wave.load(), 7);
         blocks = b.strip.nsx * b.strip.nsy;
     } else {
         b.ppc = split_patches_per_cta(a.npatches, PPB, per_wave.load());

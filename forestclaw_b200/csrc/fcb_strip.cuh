@@ -68,10 +68,10 @@ constexpr int kStripRowsMax = 2048;  // bounds a strip's tables in shared memory
 
 // Strip width and height of a mesh of n x n cells for strips of at most `most`
 // columns on a chip that holds per_wave of them at once.  A strip of h rows
-// takes h + 7 row-iterations (four ghost rows, three of pipeline), so few tall
-// strips do the least work and many short ones finish soonest: of the heights
-// that give 1, 2, ... full waves, the one whose waves x iterations is least.
-inline void strip_plan(StripArgs& g, int most, int per_wave) {
+// takes h + extra row-iterations (ghost rows, pipeline), so few tall strips do the
+// least work and many short ones finish soonest: of the heights that give 1, 2, ...
+// full waves, the one whose waves x iterations is least.
+inline void strip_plan(StripArgs& g, int most, int per_wave, int extra) {
     g.nsx = (g.n + most - 1) / most;
     g.w = (g.n + g.nsx - 1) / g.nsx;
     g.nsx = (g.n + g.w - 1) / g.w;
@@ -81,7 +81,7 @@ inline void strip_plan(StripArgs& g, int most, int per_wave) {
         const int h = std::max(std::min(g.n, 2), (g.n + nsy - 1) / nsy);
         if (h > kStripRowsMax) continue;
         const long ctas = (long)g.nsx * ((g.n + h - 1) / h);
-        const long cost = (ctas + per_wave - 1) / per_wave * (h + 7);
+        const long cost = (ctas + per_wave - 1) / per_wave * (h + extra);
         if (best < 0 || cost < best) {
             best = cost;
             g.h = h;
