@@ -96,26 +96,31 @@ __device__ __forceinline__ void physbc_op(const GhostArgs& a, const GhostOp& op,
             const bool xside = side < 2;
             const int len = xside ? ny : nx;
             const int n = meqn * mbc * len;
-            for (int k = lane; k < n; k += 32) {
-                const int m = k / (mbc * len), rem = k - m * mbc * len;
-                const int bc = rem / len + 1, t = rem % len + (1 - mbc);
-                if (side == 0) {
-                    double v = (mth == 1) ? D.at(1, t, m) : D.at(bc, t, m);
-                    if (mth == 3 && m == 1) v = -v;
-                    D.at(1 - bc, t, m) = v;
-                } else if (side == 1) {
-                    double v = (mth == 1) ? D.at(mx, t, m) : D.at(mx + 1 - bc, t, m);
-                    if (mth == 3 && m == 1) v = -v;
-                    D.at(mx + bc, t, m) = v;
-                } else if (side == 2) {
-                    double v = (mth == 1) ? D.at(t, 1, m) : D.at(t, bc, m);
-                    if (mth == 3 && m == 2) v = -v;
-                    D.at(t, 1 - bc, m) = v;
-                } else {
-                    double v = (mth == 1) ? D.at(t, my, m) : D.at(t, my + 1 - bc, m);
-                    if (mth == 3 && m == 2) v = -v;
-                    D.at(t, my + bc, m) = v;
+            // a side reads interior columns (rows) and writes ghost ones, so the loads of
+            // several cells go before their stores
+            constexpr int U = 8;
+            for (int k0 = lane; k0 < n; k0 += 32 * U) {
+                double v[U];
+                double* dst[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int k = k0 + 32 * u;
+                    dst[u] = nullptr;
+                    v[u] = 0.0;
+                    if (k < n) {
+                        const int m = k / (mbc * len), rem = k - m * mbc * len;
+                        const int bc = rem / len + 1, t = rem % len + (1 - mbc);
+                        const int g = (side & 1) ? (xside ? mx : my) + bc : 1 - bc;  // ghost column or row
+                        const int f = (side & 1) ? (mth == 1 ? (xside ? mx : my) : (xside ? mx : my) + 1 - bc)
+                                                 : (mth == 1 ? 1 : bc);
+                        v[u] = xside ? D.at(f, t, m) : D.at(t, f, m);
+                        if (mth == 3 && m == (xside ? 1 : 2)) v[u] = -v[u];
+                        dst[u] = xside ? &D.at(g, t, m) : &D.at(t, g, m);
+                    }
                 }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (dst[u]) *dst[u] = v[u];
             }
         }
         __syncwarp();
@@ -231,12 +236,19 @@ __device__ __forceinline__ double* op_cell(const GhostArgs& a, const GhostOp& op
     }
 }
 
-// One warp per group.  The records of a group share their destination patch;
+// a.wpg warps per group.  The records of a group share their destination patch;
 // the host proved every record of a wave independent of the others (none reads
 // or writes a cell another writes), so their work items may run in any order:
-// the warp lays the items of up to 32 records out in one flat index range
-// (prefix sum of op_cells over the lanes) and each lane takes items lane,
-// lane+32, ...  UNROLL items per lane issue their loads before any store.
+// a warp lays the items of up to 32 records out in one flat index range
+// (prefix sum of op_cells over the lanes) and the lanes of the group's warps take
+// items in turn.  UNROLL items per lane issue their loads before any store.
+//
+// What bounds it: the latency of a lane's dependent rounds of loads, and the bytes in
+// flight.  A wave of a refined mesh has from 1 to 2,000 groups, which at one warp each
+// leave the SMs at 13 warps or fewer; with as many warps per group as fill the chip
+// (launch_ghost_wave) the 1,870 groups of the largest wave of a shallow-water mesh
+// (levels 3-6, mx = 32) take 22.6 instead of 24.0 us from cold caches, the 320 of a small
+// one 8.3 instead of 10.0 us; what is left is the chain record -> cell -> load -> store.
 constexpr int GHOST_TPB = 256;
 template <int GHOST_UNROLL, int MXC>
 __global__ void __launch_bounds__(GHOST_TPB) ghost_wave_kernel(const GhostArgs a) {
@@ -245,8 +257,10 @@ __global__ void __launch_bounds__(GHOST_TPB) ghost_wave_kernel(const GhostArgs a
     const int wl = threadIdx.x >> 5;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (warp >= a.ngroups) return;
-    const int b = a.groups[warp], e = a.groups[warp + 1];
+    const int group = warp >> a.wpg_log2, sub = warp & ((1 << a.wpg_log2) - 1);
+    if (group >= a.ngroups) return;
+    const int step = 32 << a.wpg_log2;  // items the group's warps take at a time
+    const int b = a.groups[group], e = a.groups[group + 1];
     for (int base = b; base < e; base += 32) {
         const int cnt = min(32, e - base);
         int n = 0;
@@ -267,12 +281,12 @@ __global__ void __launch_bounds__(GHOST_TPB) ghost_wave_kernel(const GhostArgs a
         const int total = __shfl_sync(0xffffffffu, incl, 31);
         __syncwarp();
         int r = 0;  // record of the current item; items are visited in increasing order
-        for (int f0 = lane; f0 < total; f0 += 32 * GHOST_UNROLL) {
+        for (int f0 = 32 * sub + lane; f0 < total; f0 += step * GHOST_UNROLL) {
             double v[GHOST_UNROLL];
             double* dst[GHOST_UNROLL];
 #pragma unroll
             for (int u = 0; u < GHOST_UNROLL; ++u) {
-                const int f = f0 + 32 * u;
+                const int f = f0 + step * u;
                 dst[u] = nullptr;
                 v[u] = 0.0;
                 if (f < total) {
@@ -286,7 +300,7 @@ __global__ void __launch_bounds__(GHOST_TPB) ghost_wave_kernel(const GhostArgs a
                 if (dst[u]) *dst[u] = v[u];
         }
         // physical-boundary records (independent of the items above)
-        unsigned pm = __ballot_sync(0xffffffffu, phys);
+        unsigned pm = sub == 0 ? __ballot_sync(0xffffffffu, phys) : 0u;
         while (pm) {
             const int l = __ffs(pm) - 1;
             pm &= pm - 1;
@@ -309,9 +323,13 @@ void launch_ghost_shape(const GhostArgs& a, cudaStream_t st, int unroll, int blo
 }
 }  // namespace
 
-cudaError_t launch_ghost_wave(const GhostArgs& a, cudaStream_t st, int unroll) {
-    if (a.ngroups <= 0) return cudaSuccess;
-    const int blocks = (int)(((int64_t)a.ngroups * 32 + GHOST_TPB - 1) / GHOST_TPB);
+cudaError_t launch_ghost_wave(const GhostArgs& a0, cudaStream_t st, int unroll) {
+    if (a0.ngroups <= 0) return cudaSuccess;
+    // warps per group (1 to 8): about 32 warps per SM of 148
+    GhostArgs a = a0;
+    a.wpg_log2 = 0;
+    while (a.wpg_log2 < 3 && ((int64_t)a.ngroups << (a.wpg_log2 + 1)) <= 148 * 32) ++a.wpg_log2;
+    const int blocks = (int)(((((int64_t)a.ngroups) << a.wpg_log2) * 32 + GHOST_TPB - 1) / GHOST_TPB);
     const int shape = (a.mbc == 2 && a.mx == a.my) ? a.mx : 0;
     switch (shape) {
         case 8: launch_ghost_shape<8>(a, st, unroll, blocks); break;
@@ -327,6 +345,9 @@ cudaError_t launch_ghost_wave(const GhostArgs& a, cudaStream_t st, int unroll) {
 // Time interpolation on the interior band of width mbc (the four strips in the
 // reference's order; every strip cell is written once, so order is free).
 // ---------------------------------------------------------------------------
+// One CTA per patch.  Bound by latency: only the cells of the mbc-deep band inside the
+// patch, which is all that a finer neighbour reads, are enumerated; scanning the whole
+// interior for them took 19 us per 100 patches of 32 x 32 (three fields), this 5.5 us.
 __global__ void timeinterp_kernel(double* q, const double* qlast, double* qti, int64_t stride,
                                   const int32_t* slots, int n, int mx, int my, int mbc, int meqn,
                                   double alpha) {
@@ -334,13 +355,21 @@ __global__ void timeinterp_kernel(double* q, const double* qlast, double* qti, i
     if (p >= n) return;
     const int64_t base = (int64_t)slots[p] * stride;
     const int nx = mx + 2 * mbc, ny = my + 2 * mbc;
-    const int mint = mbc;
-    const int total = meqn * mx * my;
-    for (int k = threadIdx.x; k < total; k += blockDim.x) {
-        const int m = k / (mx * my), rem = k - m * mx * my;
-        const int j = rem / mx + 1, i = rem % mx + 1;
-        const bool in_band = (i <= mint) || (i > mx - mint) || (j <= mint) || (j > my - mint);
-        if (!in_band) continue;
+    // the band's cells, mbc deep: whole rows at the bottom and top, then the column
+    // ends of the rows between
+    const int rows = 2 * mbc * mx, cols = 2 * mbc * (my - 2 * mbc), per = rows + cols;
+    for (int k = threadIdx.x; k < meqn * per; k += blockDim.x) {
+        const int m = k / per, e = k - m * per;
+        int i, j;
+        if (e < rows) {
+            const int r = e / mx;
+            i = e - r * mx + 1;
+            j = r < mbc ? r + 1 : my - 2 * mbc + r + 1;
+        } else {
+            const int r = (e - rows) / (2 * mbc), w = (e - rows) - r * 2 * mbc;
+            i = w < mbc ? w + 1 : mx - 2 * mbc + w + 1;
+            j = mbc + r + 1;
+        }
         const int64_t idx = base + ((int64_t)m * ny + (j + mbc - 1)) * nx + (i + mbc - 1);
         qti[idx] = qlast[idx] + alpha * (q[idx] - qlast[idx]);
     }
@@ -350,7 +379,7 @@ cudaError_t launch_timeinterp(double* q, const double* qlast, double* qti, int64
                               const int32_t* slots, int n, int mx, int my, int mbc, int meqn,
                               double alpha, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    timeinterp_kernel<<<n, 128, 0, st>>>(q, qlast, qti, stride, slots, n, mx, my, mbc, meqn, alpha);
+    timeinterp_kernel<<<n, 256, 0, st>>>(q, qlast, qti, stride, slots, n, mx, my, mbc, meqn, alpha);
     return cudaGetLastError();
 }
 
