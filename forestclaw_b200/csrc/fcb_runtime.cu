@@ -243,7 +243,8 @@ PartitionPlan Context::partition_plan(const fcb_options_t& o, const std::vector<
     const int n = (int)leaves.size();
     try {
         c.nbrs_.resize(n);
-        for (int p = 0; p < n; ++p) c.nbrs_[p] = c.forest_.neighbors(p);
+        const QuadForest::Locator at(c.forest_);
+        for (int p = 0; p < n; ++p) c.nbrs_[p] = c.forest_.neighbors(p, at);
     } catch (const std::runtime_error& e) {
         throw Error(FCB_ERR_INVALID, std::string("leaves: ") + e.what());
     }
@@ -258,7 +259,9 @@ PartitionPlan Context::partition_plan(const fcb_options_t& o, const std::vector<
     out.first = c.own_first_;
     out.count = c.own_count_;
     out.ghosts = k - c.own_count_;
-    const PlanBuild b = c.build_plan(minlevel, maxlevel, ti);
+    PlanWork w;
+    c.build_plan(minlevel, maxlevel, ti, w);
+    const PlanBuild& b = w.built;
     out.x1_send = b.x1.send_n;
     out.x1_recv = b.x1.recv_n;
     out.x2_send = b.x2.send_n;
@@ -391,13 +394,15 @@ PatchMeta Context::meta_of(const Leaf& l) const {
 }
 
 // Neighbour relations of every leaf (point location in the Morton-sorted
-// leaves), split over host threads for large forests.
+// leaves), split over host threads for large forests: 4,096 leaves take 0.5 ms,
+// a thread's start about 0.03 ms.
 void Context::compute_neighbors() {
     const int n = num_patches();
     nbrs_.resize(n);
-    const int nt = (int)std::min<unsigned>({8u, std::max(1u, std::thread::hardware_concurrency()), (unsigned)(n / 512 + 1)});
+    const QuadForest::Locator at(forest_);
+    const int nt = (int)std::min<unsigned>({8u, std::max(1u, std::thread::hardware_concurrency()), (unsigned)(n / 4096 + 1)});
     if (nt == 1) {
-        for (int p = 0; p < n; ++p) nbrs_[p] = forest_.neighbors(p);
+        for (int p = 0; p < n; ++p) nbrs_[p] = forest_.neighbors(p, at);
         return;
     }
     std::vector<std::thread> ts;
@@ -406,7 +411,7 @@ void Context::compute_neighbors() {
         ts.emplace_back([&, k] {
             try {
                 for (int p = (int)((int64_t)n * k / nt); p < (int)((int64_t)n * (k + 1) / nt); ++p)
-                    nbrs_[p] = forest_.neighbors(p);
+                    nbrs_[p] = forest_.neighbors(p, at);
             } catch (...) {
                 err[k] = std::current_exception();
             }
@@ -492,18 +497,6 @@ void Context::mesh_changed() {
 // ---------------------------------------------------------------------------
 // Ghost plans
 // ---------------------------------------------------------------------------
-namespace {
-struct Rect {
-    int i0, i1, j0, j1;
-    bool hits(const Rect& o) const { return i0 <= o.i1 && o.i0 <= i1 && j0 <= o.j1 && o.j0 <= j1; }
-};
-struct Touch {
-    int64_t key;  // slot * 2 + time-interp array
-    Rect r;
-    bool write;
-};
-}  // namespace
-
 // fclaw2d_ghost_update_async (src/fclaw2d_ghost_fill.c:611-831) on one rank:
 // the records are emitted in the order the reference's callbacks run.
 void Context::build_ops(int minlevel, int maxlevel, int ti, std::vector<GhostOp>& ops, size_t* phase_b) const {
@@ -511,6 +504,9 @@ void Context::build_ops(int minlevel, int maxlevel, int ti, std::vector<GhostOp>
     const int n = num_patches();
     std::vector<std::vector<int>> at((size_t)QuadForest::kMaxLevel + 1);
     for (int p = 0; p < n; ++p) at[forest_.leaves[p].level].push_back(p);
+    size_t used = 0;
+    for (int l = std::max(0, minlevel - 1); l <= std::min(maxlevel, QuadForest::kMaxLevel); ++l) used += at[l].size();
+    ops.reserve(10 * used);
     auto level_list = [&](int l) -> const std::vector<int>& {
         static const std::vector<int> empty;
         return (l < 0 || l > QuadForest::kMaxLevel) ? empty : at[l];
@@ -614,18 +610,21 @@ void Context::build_ops(int minlevel, int maxlevel, int ti, std::vector<GhostOp>
 // so the first set reads only source interiors as they were before the update,
 // and the second reads sources as the first set left them: sending those two
 // states of the other ranks' patches reproduces the one-rank order exactly.
-Context::PlanBuild Context::build_plan(int minlevel, int maxlevel, int ti) const {
-    std::vector<GhostOp> ops;
+void Context::build_plan(int minlevel, int maxlevel, int ti, PlanWork& w) const {
+    std::vector<GhostOp>& ops = w.ops;
+    ops.clear();
     size_t phase_b = 0;
     build_ops(minlevel, maxlevel, ti, ops, &phase_b);
+    PlanBuild& b = w.built;
+    b.x1 = b.x2 = XList{};
     if (!partitioned()) {
         for (GhostOp& o : ops) {
             o.dst = slot_of_[o.dst];
             o.src = slot_of_[o.src];
         }
-        PlanBuild b = make_waves(ops);
+        make_waves(ops, w, b);
         b.nA = (int)b.wave_begin.size() - 1;
-        return b;
+        return;
     }
     // exchange items (leaf * 2 + array) this rank receives from / sends to each rank
     const int R = nranks_;
@@ -652,9 +651,10 @@ Context::PlanBuild Context::build_plan(int minlevel, int maxlevel, int ti) const
         if (o.dst < 0 || o.src < 0) throw Error(FCB_ERR_INTERNAL, "ghost record outside the local patches");
         mine[x].push_back(o);
     }
-    PlanBuild b = make_waves(mine[0]);
+    make_waves(mine[0], w, b);
     b.nA = (int)b.wave_begin.size() - 1;
-    PlanBuild c = make_waves(mine[1]);
+    PlanBuild c;
+    make_waves(mine[1], w, c);
     const int nops = (int)b.ops.size(), ngroups = (int)b.groups.size();
     b.ops.insert(b.ops.end(), c.ops.begin(), c.ops.end());
     for (size_t w = 1; w < c.wave_begin.size(); ++w) b.wave_begin.push_back(c.wave_begin[w] + nops);
@@ -681,31 +681,35 @@ Context::PlanBuild Context::build_plan(int minlevel, int maxlevel, int ti) const
             xl.recv_n[r] = (int)recv[x][r].size();
         }
     }
-    return b;
 }
 
 // Records in waves: each record goes one wave after the latest earlier record
 // it conflicts with (read-after-write, write-after-read, write-after-write on
 // overlapping cells of the same array), so the records of a wave are
 // independent and the waves keep the reference's order.
-Context::PlanBuild Context::make_waves(const std::vector<GhostOp>& ops) const {
+void Context::make_waves(const std::vector<GhostOp>& ops, PlanWork& work, PlanBuild& b) const {
+    using Rect = PlanRect;
+    struct Touch {
+        int64_t key;  // slot * 2 + time-interp array
+        Rect r;
+        bool write;
+    };
     const int mx = opt_.mx, my = opt_.my, mbc = opt_.mbc;
     const Rect whole{1 - mbc, mx + mbc, 1 - mbc, my + mbc};
     const Rect interior{1, mx, 1, my};
-    std::vector<int> wave(ops.size(), 0);
-    // writes and reads seen so far, per array (slot * 2 + time-interp flag):
-    // a read conflicts only with writes, a write with both.  Each array's
-    // touches form a list through flat arrays (newest first), no allocation
-    // per array.
+    std::vector<int>& wave = work.wave;
+    wave.assign(ops.size(), 0);
+    // Touches seen so far, per array (slot * 2 + time-interp flag): a read conflicts
+    // only with writes, a write with both.  Only a physical boundary (the whole array)
+    // and ghost regions are written, so a read inside the interior, the commonest
+    // touch, conflicts with the former alone and a number per array settles it; the
+    // touches of ghost regions form lists through a flat array (newest first).
     const size_t narr = (size_t)2 * std::max(1, capacity_);
-    struct Seen {
-        Rect r;
-        int wave;
-        int next;
-    };
-    std::vector<Seen> seen;
-    seen.reserve(2 * ops.size());
-    std::vector<int> head_w(narr, -1), head_r(narr, -1);
+    std::vector<PlanTouch>& seen = work.seen;
+    seen.clear();
+    std::vector<PlanArray>& arrays = work.arrays;
+    arrays.assign(narr, PlanArray{});
+    auto inside = [&](const Rect& r) { return r.i0 >= 1 && r.i1 <= mx && r.j0 >= 1 && r.j1 <= my; };
     auto band = [&](int face) -> Rect {
         if (face == 0) return {1 - mbc, 0, 1, my};
         if (face == 1) return {mx + 1, mx + mbc, 1, my};
@@ -761,22 +765,35 @@ Context::PlanBuild Context::make_waves(const std::vector<GhostOp>& ops) const {
                 break;
         }
         int w = 0;
+        const bool all = o.type == OP_PHYSBC;
         for (const Touch& a : t) {
-            for (int i = head_w[(size_t)a.key]; i >= 0; i = seen[i].next)
-                if (seen[i].wave >= w && a.r.hits(seen[i].r)) w = seen[i].wave + 1;
-            if (a.write)
-                for (int i = head_r[(size_t)a.key]; i >= 0; i = seen[i].next)
+            const PlanArray& y = arrays[(size_t)a.key];
+            w = std::max(w, y.w_whole + 1);
+            if (all || (a.write && a.r.hits(interior))) {  // as if it touched the whole array
+                w = std::max(w, y.w_all + 1);
+                if (a.write) w = std::max(w, y.r_all + 1);
+            } else if (a.write || !inside(a.r)) {
+                for (int i = y.head_w; i >= 0; i = seen[i].next)
                     if (seen[i].wave >= w && a.r.hits(seen[i].r)) w = seen[i].wave + 1;
+                if (a.write)
+                    for (int i = y.head_r; i >= 0; i = seen[i].next)
+                        if (seen[i].wave >= w && a.r.hits(seen[i].r)) w = seen[i].wave + 1;
+            }
         }
         wave[k] = w;
         for (const Touch& a : t) {
-            int& h = (a.write ? head_w : head_r)[(size_t)a.key];
-            seen.push_back({a.r, w, h});
-            h = (int)seen.size() - 1;
+            PlanArray& y = arrays[(size_t)a.key];
+            (a.write ? y.w_all : y.r_all) = std::max(a.write ? y.w_all : y.r_all, w);
+            if (all || (a.write && a.r.hits(interior))) {
+                y.w_whole = std::max(y.w_whole, w);
+            } else if (a.write || !inside(a.r)) {
+                int& h = a.write ? y.head_w : y.head_r;
+                seen.push_back({a.r, w, h});
+                h = (int)seen.size() - 1;
+            }
         }
     }
     const int nw = ops.empty() ? 0 : *std::max_element(wave.begin(), wave.end()) + 1;
-    PlanBuild b;
     b.wave_begin.assign(nw + 1, 0);
     std::vector<int> count(nw, 0);
     for (int w : wave) ++count[w];
@@ -785,9 +802,11 @@ Context::PlanBuild Context::make_waves(const std::vector<GhostOp>& ops) const {
     // among equal keys: a stable counting sort by destination slot, then a
     // stable counting sort by wave
     const size_t n = ops.size();
-    std::vector<int> by_dst(n);
+    std::vector<int>& by_dst = work.by_dst;
+    by_dst.resize(n);
     {
-        std::vector<int> start((size_t)std::max(1, capacity_) + 1, 0);
+        std::vector<int>& start = work.start;
+        start.assign((size_t)std::max(1, capacity_) + 1, 0);
         for (const GhostOp& o : ops) {
             if (o.dst < 0 || o.dst >= std::max(1, capacity_)) throw Error(FCB_ERR_INTERNAL, "ghost record outside the arena");
             ++start[(size_t)o.dst + 1];
@@ -800,6 +819,7 @@ Context::PlanBuild Context::make_waves(const std::vector<GhostOp>& ops) const {
     for (int k : by_dst) b.ops[pos[wave[k]]++] = ops[k];
     // within a wave, records with the same destination patch form one group
     b.group_begin.assign(nw + 1, 0);
+    b.groups.clear();
     for (int w = 0; w < nw; ++w) {
         b.group_begin[w] = (int)b.groups.size();
         for (int k = b.wave_begin[w]; k < b.wave_begin[w + 1]; ++k)
@@ -807,15 +827,34 @@ Context::PlanBuild Context::make_waves(const std::vector<GhostOp>& ops) const {
         b.groups.push_back(b.wave_begin[w + 1]);  // end marker of the wave
     }
     b.group_begin[nw] = (int)b.groups.size();
-    return b;
 }
 
-const GhostPlan& Context::commit_plan(const std::tuple<int, int, int>& key, PlanBuild&& b) {
+size_t Context::PlanWork::bytes() const {
+    return (ops.capacity() + built.ops.capacity()) * sizeof(GhostOp) + seen.capacity() * sizeof(PlanTouch) +
+           arrays.capacity() * sizeof(PlanArray) +
+           (wave.capacity() + by_dst.capacity() + start.capacity() + built.groups.capacity()) * sizeof(int);
+}
+
+Context::PlanWork& Context::plan_work(size_t k) {
+    while (plan_work_.size() <= k) plan_work_.emplace_back(std::make_unique<PlanWork>());
+    return *plan_work_[k];
+}
+
+// Keeps at most 64 MB of build memory (meshes of about 20,000 patches).
+void Context::trim_plan_work() {
+    size_t kept = 0;
+    for (auto& w : plan_work_) {
+        kept += w->bytes();
+        if (kept > ((size_t)64 << 20)) *w = PlanWork{};
+    }
+}
+
+const GhostPlan& Context::commit_plan(const std::tuple<int, int, int>& key, PlanBuild& b) {
     GhostPlan g;
     g.first = h_ops_.size();
     g.first_group = h_groups_.size();
-    g.wave_begin = std::move(b.wave_begin);
-    g.group_begin = std::move(b.group_begin);
+    g.wave_begin = b.wave_begin;
+    g.group_begin = b.group_begin;
     for (int32_t k : b.groups) h_groups_.push_back((int32_t)(g.first + k));
     h_ops_.insert(h_ops_.end(), b.ops.begin(), b.ops.end());
     g.nA = b.nA;
@@ -843,7 +882,11 @@ const GhostPlan& Context::plan(int minlevel, int maxlevel, int ti) {
         it = plans_.find(key);
         if (it != plans_.end()) return it->second;
     }
-    return commit_plan(key, build_plan(minlevel, maxlevel, ti));
+    PlanWork& w = plan_work(0);
+    build_plan(minlevel, maxlevel, ti, w);
+    const GhostPlan& g = commit_plan(key, w.built);
+    trim_plan_work();
+    return g;
 }
 
 void Context::start_plans(const std::vector<std::tuple<int, int, int>>& keys) {
@@ -852,14 +895,14 @@ void Context::start_plans(const std::vector<std::tuple<int, int, int>>& keys) {
         if (!plans_.count(k) && std::find(plan_todo_.begin(), plan_todo_.end(), k) == plan_todo_.end())
             plan_todo_.push_back(k);
     if (plan_todo_.empty()) return;
-    plan_built_.assign(plan_todo_.size(), PlanBuild{});
+    plan_work(plan_todo_.size() - 1);
     plan_err_.assign(plan_todo_.size(), nullptr);
     // the builds only read the forest, neighbour tables, slot map and options
     for (size_t k = 0; k < plan_todo_.size(); ++k)
         plan_threads_.emplace_back([this, k] {
             try {
                 const auto& t = plan_todo_[k];
-                plan_built_[k] = build_plan(std::get<0>(t), std::get<1>(t), std::get<2>(t));
+                build_plan(std::get<0>(t), std::get<1>(t), std::get<2>(t), *plan_work_[k]);
             } catch (...) {
                 plan_err_[k] = std::current_exception();
             }
@@ -895,7 +938,6 @@ void Context::prefetch_plans() {
 void Context::discard_plans() noexcept {
     join_plans();
     plan_todo_.clear();
-    plan_built_.clear();
     plan_err_.clear();
 }
 
@@ -914,11 +956,11 @@ void Context::finish_plans() {
             if (!err) err = plan_err_[k];
             continue;
         }
-        if (!plans_.count(plan_todo_[k])) commit_plan(plan_todo_[k], std::move(plan_built_[k]));
+        if (!plans_.count(plan_todo_[k])) commit_plan(plan_todo_[k], plan_work_[k]->built);
     }
     plan_todo_.clear();
-    plan_built_.clear();
     plan_err_.clear();
+    trim_plan_work();
     if (err) std::rethrow_exception(err);
 }
 
@@ -2462,7 +2504,7 @@ bool Context::adapt(const std::vector<int>& target, std::vector<Leaf>& out) {
 
 void Context::qinit_slots(const std::vector<int32_t>& slots) {
     if (slots.empty()) return;
-    DevBuf<int32_t> d;
+    DevBuf<int32_t>& d = d_xfer_;  // only grows: a freed buffer would synchronise the whole device
     d.reserve(slots.size());
     check(cudaMemcpy(d.p, slots.data(), slots.size() * 4, cudaMemcpyHostToDevice), "qinit slots");
     QinitArgs a{};
@@ -2795,9 +2837,12 @@ void Context::initialize() {
             const std::vector<int> old_slots = slot_of_;
             const std::vector<int> old_owner = owner_;
             forest_.leaves = nl;
-            if (partitioned()) repopulate_partitioned(old, old_slots, old_owner, true);
-            else repopulate(old, old_slots, true);
-            mesh_changed();
+            if (partitioned()) {
+                repopulate_partitioned(old, old_slots, old_owner, true);
+                mesh_changed();
+            } else {
+                repopulate(old, old_slots, true);  // calls mesh_changed before it fills the patches
+            }
         }
     }
     if (opt_.init_ghostcell) ghost_update(forest_.min_level(), forest_.max_level(), 0.0, 0);

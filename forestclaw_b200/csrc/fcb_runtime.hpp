@@ -210,9 +210,35 @@ class Context {
         int nA = 0;
         XList x1, x2;
     };
-    PlanBuild build_plan(int minlevel, int maxlevel, int time_interp) const;
-    PlanBuild make_waves(const std::vector<GhostOp>& ops) const;
-    const GhostPlan& commit_plan(const std::tuple<int, int, int>& key, PlanBuild&& b);
+    struct PlanRect {
+        int i0, i1, j0, j1;
+        bool hits(const PlanRect& o) const { return i0 <= o.i1 && o.i0 <= i1 && j0 <= o.j1 && o.j0 <= j1; }
+    };
+    struct PlanTouch {  // a touch of a ghost region, in its array's list
+        PlanRect r;
+        int wave;
+        int next;
+    };
+    struct PlanArray {
+        int w_whole = -1;            // latest wave that touches the whole array
+        int w_all = -1, r_all = -1;  // latest wave that writes / reads any of it
+        int head_w = -1, head_r = -1;
+    };
+    // The memory of one plan build, kept from mesh to mesh: arrays of this size come
+    // from mmap, and faulting fresh pages in took as long as the build itself.
+    struct PlanWork {
+        std::vector<GhostOp> ops;
+        std::vector<int> wave, by_dst, start;
+        std::vector<PlanTouch> seen;
+        std::vector<PlanArray> arrays;
+        PlanBuild built;
+        size_t bytes() const;
+    };
+    void build_plan(int minlevel, int maxlevel, int time_interp, PlanWork& w) const;  // into w.built
+    void make_waves(const std::vector<GhostOp>& ops, PlanWork& w, PlanBuild& b) const;
+    const GhostPlan& commit_plan(const std::tuple<int, int, int>& key, PlanBuild& b);
+    PlanWork& plan_work(size_t k);  // the k-th build's memory
+    void trim_plan_work();
     // Missing plans of a macro step are built on host threads while its first
     // level updates run on the GPU; plan() waits for them.  Every build ends
     // (finish_plans) before advance_all_levels returns, so no build outlives a
@@ -251,7 +277,7 @@ class Context {
     int32_t* h_ts_groups_pinned_ = nullptr;
     size_t h_ts_groups_pinned_cap_ = 0;
     std::vector<std::tuple<int, int, int>> plan_todo_;
-    std::vector<PlanBuild> plan_built_;
+    std::vector<std::unique_ptr<PlanWork>> plan_work_;  // one per build that runs at once
     std::vector<std::exception_ptr> plan_err_;
     std::vector<std::thread> plan_threads_;
     // pinned staging of the op and group buffers, and the event of its last upload
