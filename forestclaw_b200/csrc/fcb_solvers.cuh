@@ -1066,7 +1066,18 @@ __device__ __forceinline__ void limiter_values(const R* num, const R* wn2, const
 #pragma unroll
         for (int mw = 0; mw < W; ++mw) {
             const int mth = lim(mw);
-            const R p = limiter_phi((V5 && mth > 5) ? 1 : mth, r[mw]);
+            R p;
+            if (mth == 3) {  // van Leer: the quotient without branches
+                bool ok3 = true;
+                const Dv<R> d(R(1.0) + fabs(r[mw]), ok3);
+                p = d(r[mw] + fabs(r[mw]), ok3);
+                if (!ok3) {
+                    seldom();
+                    p = limiter_phi(3, r[mw]);
+                }
+            } else {
+                p = limiter_phi((V5 && mth > 5) ? 1 : mth, r[mw]);
+            }
             phi[mw] = (mth == 0 || wn2[mw] == R(0)) ? R(1) : p;
         }
     }

@@ -40,7 +40,7 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* p, double 
     atomicMax(p, (unsigned long long)__double_as_longlong(v));
 }
 
-template <int NX, int NY, int PPB, int M, int W, int NAUX, bool PSI, int NC>
+template <int NX, int NY, int PPB, int M, int W, int NAUX, bool PSI, int NC, bool CAPA>
 struct StepSmem {
     static constexpr int QROW = 0;
     static constexpr int XW = QROW + 3 * PPB * NX * M;
@@ -49,7 +49,8 @@ struct StepSmem {
     static constexpr int FX = GL + PPB * NX * 2 * M;
     static constexpr int GY = FX + 3 * PPB * NX * 2 * M;
     static constexpr int CROW = GY + PPB * NX * 2 * M;
-    static constexpr int GXR = CROW + 2 * PPB * NX * NC;
+    static constexpr int DTX = CROW + 2 * PPB * NX * NC;
+    static constexpr int GXR = DTX + (CAPA ? PPB * NX : 0);
     static constexpr int AUX = GXR + 3 * PPB * NX * M;
     static constexpr int TAB = AUX + PPB * NAUX * NY * NX;
     static constexpr int PSIT = TAB + (PSI ? PPB * 2 * (NX + 1) : 0);
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
     constexpr int NX = MX + 2 * MBC;
     constexpr int NY = NX;
     constexpr int PPB = TPB / NX;
-    using L = StepSmem<NX, NY, PPB, M, W, NAUX, AUXK == AUX_SWIRL, NC>;
+    using L = StepSmem<NX, NY, PPB, M, W, NAUX, AUXK == AUX_SWIRL, NC, AuxLayout<SOL>::CAPA>;
     using Cell = typename SOL::Cell;
     // mapped grids: the Riemann solvers read aux from component KS on, and
     // aux(1) is the capacity kappa (dtdx1d(i) = dtdx / kappa(i), clawpack46_step2.f:122-126)
@@ -90,7 +91,6 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
     // clawpack5_step2_wrap.f updates the interior cells 1..mx, 1..my only;
     // those read the interfaces 1..mx+1, whose fluxes are the same as 4.6's
     constexpr bool V5 = SOL::V5;
-    auto LIMV = [](int l) { return (V5 && l > 5) ? 1 : l; };
     const MethodC<LIM> meth{a};
     extern __shared__ double smem[];
     double* s_qrow = smem + L::QROW;  // [3][PPB][NX][M]: rows s-2, s-1, s (slot row % 3)
@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
     double* s_fx = smem + L::FX;      // [3][PPB][NX][2][M]
     double* s_gy = smem + L::GY;      // [PPB][NX][2][M]
     double* s_crow = smem + L::CROW;  // [2][PPB][NX][NC]: the cell quantities of rows s-1 and s
+    double* s_dtx = smem + L::DTX;    // [PPB][NX]: dtdx / kappa of row s (capacity)
     double* s_gxr = smem + L::GXR;    // [3][PPB][NX][M]: GXu(row-1) + GXd(row) of rows s-2, s-1, s (own column)
     double* s_aux = smem + L::AUX;    // [PPB][NAUX][NY][NX]
     double* s_tab = smem + L::TAB;    // [PPB][2][NX+1] (swirl)
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
         if (active) {
             const double* ag = D ? D->aux : a.aux + (int64_t)slot * a.aux_stride;
             for (int k = 0; k < NAUX; ++k)
+#pragma unroll 12
                 for (int r = 0; r < NY; ++r)
                     s_aux[((pl * NAUX + k) * NY + r) * NX + c] = ag[(k * NY + r) * NX + c];
         }
@@ -200,15 +202,15 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
         if constexpr (NAUX > 0) return s_aux[((pl * NAUX + k) * NY + rr) * NX + cc];
         else return 0.0;
     };
-    // dtdx1d / dtdy1d of cell (cc, rr)
-    auto DTDX = [&](int cc, int rr) -> double {
-        if constexpr (CAPA) return dtdx / AUXV(0, cc, rr);
-        else return dtdx;
-    };
-    auto DTDY = [&](int cc, int rr) -> double {
-        if constexpr (CAPA) return dtdy / AUXV(0, cc, rr);
-        else return dtdy;
-    };
+    // Capacity: the three quotients of a cell with its kappa (dtdx1d, dtdy1d and the
+    // update's) share one reciprocal, taken when its row arrives and kept for the two
+    // rows that follow: ty = dtdy / kappa, ky = the reciprocal, kok = in the method's
+    // range, of rows s, s-1 and s-2.  (Seven divisions a cell, one after another, held
+    // 226 CTAs of three 32 x 32 patches, 1.5 per SM and bound by latency, at 151 us;
+    // with this and the row loaded ahead 115 us.)
+    double ty_n = dtdy, ty_1 = dtdy, ty_2 = dtdy, tx_n = dtdx;
+    [[maybe_unused]] double ky_n = 0.0, ky_1 = 0.0, ky_2 = 0.0;
+    [[maybe_unused]] bool kok_n = false, kok_1 = false, kok_2 = false;
 
     const bool ycol = active && c >= 1 && c <= NX - 2;
     double cfl = 0.0;
@@ -252,15 +254,39 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
         return reinterpret_cast<Cell*>(s_crow + (((rr & 1) * PPB + pl) * NX + cc) * NC);
     };
 
+    // scalar equations: a row is loaded one row ahead
+    [[maybe_unused]] double q_ahead = 0.0;
+    if constexpr (M == 1)
+        if (active) q_ahead = qin[(int64_t)s0 * NX + c];
     for (int s = s0; s <= s1; ++s) {
         // ---------------- phase 1: load row s; raw y-interface s ----------------
         if (s < NY && active) {
 #pragma unroll
             for (int m = 0; m < M; ++m) {
                 const int64_t k = ((int64_t)m * NY + s) * NX + c;
-                q_n[m] = qin[k];
+                if constexpr (M == 1) {
+                    q_n[m] = q_ahead;
+                    if (s + 1 < NY) q_ahead = qin[k + NX];
+                } else {
+                    q_n[m] = qin[k];
+                }
                 if (save_last && s >= qlo && s < qhi) qlast[k] = q_n[m];
                 QR(s, c)[m] = q_n[m];
+            }
+            if constexpr (CAPA) {
+                bool ok = true;
+                const double kappa = AUXV(0, c, s);
+                const Dv<double> d(kappa, ok);
+                ky_n = d.y;
+                kok_n = ok;
+                tx_n = d(dtdx, ok);
+                ty_n = d(dtdy, ok);
+                if (!ok) {
+                    seldom();
+                    tx_n = dtdx / kappa;
+                    ty_n = dtdy / kappa;
+                }
+                s_dtx[pl * NX + c] = tx_n;
             }
             Cell cn;
             sol.prep(q_n, cn);
@@ -291,7 +317,7 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
 #pragma unroll
                 for (int m = 0; m < M; ++m) w[mw][m] = yw_f[mw][m];
             // dtdy1d of the cells below (f-1) and above (f) the interface
-            const double dty_lo = DTDY(c, f - 1), dty_hi = DTDY(c, f);
+            const double dty_lo = ty_2, dty_hi = ty_1;
             if (f >= MBC && f <= MBC + MX) {
 #pragma unroll
                 for (int mw = 0; mw < W; ++mw) cfl = nanmax(nanmax(cfl, dty_hi * ys_f[mw]), -dty_lo * ys_f[mw]);
@@ -302,18 +328,19 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
             for (int m = 0; m < M; ++m) cq[m] = 0.0;
             if (meth.second_order()) {
                 if (f >= MBC && f <= MBC + MX) {
+                    double num[W], wn2[W], phi[W];
 #pragma unroll
                     for (int mw = 0; mw < W; ++mw) {
-                        if (meth.lim(mw) == 0) continue;
-                        double wn2 = yw_f[mw][0] * yw_f[mw][0];
+                        wn2[mw] = yw_f[mw][0] * yw_f[mw][0];
 #pragma unroll
-                        for (int m = 1; m < M; ++m) wn2 = wn2 + yw_f[mw][m] * yw_f[mw][m];
-                        if (wn2 == 0.0) continue;
-                        const double r = (ys_f[mw] > 0.0) ? ydotl[mw] / wn2 : ydotr[mw] / wn2;
-                        const double phi = limiter_phi(LIMV(meth.lim(mw)), r);
-#pragma unroll
-                        for (int m = 0; m < M; ++m) w[mw][m] = phi * w[mw][m];
+                        for (int m = 1; m < M; ++m) wn2[mw] = wn2[mw] + yw_f[mw][m] * yw_f[mw][m];
+                        num[mw] = (ys_f[mw] > 0.0) ? ydotl[mw] : ydotr[mw];
                     }
+                    limiter_values<V5, W>(num, wn2, [&](int mw) { return meth.lim(mw); }, phi);
+#pragma unroll
+                    for (int mw = 0; mw < W; ++mw)
+#pragma unroll
+                        for (int m = 0; m < M; ++m) w[mw][m] = phi[mw] * w[mw][m];
                 }
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
@@ -398,8 +425,8 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
         // dtdx1d of the cells left (c-1) and right (c) of the interface
         double dtx_lo = dtdx, dtx_hi = dtdx;
         if (xint) {
-            dtx_lo = DTDX(c - 1, s);
-            dtx_hi = DTDX(c, s);
+            if constexpr (CAPA) dtx_lo = s_dtx[pl * NX + c - 1];
+            dtx_hi = tx_n;
             double qL[M];
 #pragma unroll
             for (int m = 0; m < M; ++m) qL[m] = QR(s, c - 1)[m];
@@ -427,25 +454,26 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
             for (int m = 0; m < M; ++m) cq[m] = 0.0;
             if (meth.second_order()) {
                 if (c >= MBC && c <= MBC + MX) {
+                    double num[W], wn2[W], phi[W];
 #pragma unroll
                     for (int mw = 0; mw < W; ++mw) {
-                        if (meth.lim(mw) == 0) continue;
-                        double wn2 = xwl[mw][0] * xwl[mw][0];
+                        wn2[mw] = xwl[mw][0] * xwl[mw][0];
                         double dl = xw[((c - 1) * W + mw) * M + 0] * xwl[mw][0];
                         double dr = xwl[mw][0] * xw[((c + 1) * W + mw) * M + 0];
 #pragma unroll
                         for (int m = 1; m < M; ++m) {
                             const double wc = xwl[mw][m];
-                            wn2 = wn2 + wc * wc;
+                            wn2[mw] = wn2[mw] + wc * wc;
                             dl = dl + xw[((c - 1) * W + mw) * M + m] * wc;
                             dr = dr + wc * xw[((c + 1) * W + mw) * M + m];
                         }
-                        if (wn2 == 0.0) continue;
-                        const double r = (xsl[mw] > 0.0) ? dl / wn2 : dr / wn2;
-                        const double phi = limiter_phi(LIMV(meth.lim(mw)), r);
-#pragma unroll
-                        for (int m = 0; m < M; ++m) xwl[mw][m] = phi * xwl[mw][m];
+                        num[mw] = (xsl[mw] > 0.0) ? dl : dr;
                     }
+                    limiter_values<V5, W>(num, wn2, [&](int mw) { return meth.lim(mw); }, phi);
+#pragma unroll
+                    for (int mw = 0; mw < W; ++mw)
+#pragma unroll
+                        for (int m = 0; m < M; ++m) xwl[mw][m] = phi[mw] * xwl[mw][m];
                 }
 #pragma unroll
                 for (int m = 0; m < M; ++m) {
@@ -543,9 +571,17 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
                 const double gmv = GXS(s - 1)[m] + FYm_cur[m];      // gm(i, j+1)
                 const double gpv = GXS(r)[m] + FYp_prev[m];         // gp(i, j)
                 double qv;
-                if constexpr (CAPA)  // clawpack46_step2_wrap.f:118-121
-                    qv = QR(r, c)[m] - (dtdx * (fmv - fpv) + dtdy * (gmv - gpv)) / AUXV(0, c, r);
-                else
+                if constexpr (CAPA) {  // clawpack46_step2_wrap.f:118-121
+                    const double flux = dtdx * (fmv - fpv) + dtdy * (gmv - gpv);
+                    const double kappa = AUXV(0, c, r);
+                    bool ok = kok_2;
+                    double upd_q = Dv<double>(kappa, ky_2)(flux, ok);
+                    if (!ok) {
+                        seldom();
+                        upd_q = flux / kappa;
+                    }
+                    qv = QR(r, c)[m] - upd_q;
+                } else
                     qv = QR(r, c)[m] - dtdx * (fmv - fpv) - dtdy * (gmv - gpv);
                 q[((int64_t)m * NY + r) * NX + c] = qv;
                 if (a.treg) {
@@ -577,6 +613,11 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
 #pragma unroll
         for (int m = 0; m < M; ++m) {
             FYp_prev[m] = FYp_cur[m];
+        }
+        if constexpr (CAPA) {
+            ty_2 = ty_1; ty_1 = ty_n;
+            ky_2 = ky_1; ky_1 = ky_n;
+            kok_2 = kok_1; kok_1 = kok_n;
         }
     }
 
@@ -638,7 +679,7 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
     constexpr int NX = MX + 2 * MBC;
     constexpr int PPB = TPB / NX;
     static_assert(PPB >= 1, "patch wider than the CTA");
-    using L = StepSmem<NX, NX, PPB, SOL::M, SOL::W, NAUX, AUXK == AUX_SWIRL, SOL::NC>;
+    using L = StepSmem<NX, NX, PPB, SOL::M, SOL::W, NAUX, AUXK == AUX_SWIRL, SOL::NC, AuxLayout<SOL>::CAPA>;
     const size_t bytes = (size_t)L::TOTAL * sizeof(double);
     static bool configured = false;
     if (!configured) {
