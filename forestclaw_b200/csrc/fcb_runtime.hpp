@@ -319,8 +319,8 @@ class Context {
     // ensure_ghosts() before anything reads ghost cells.
     bool fusion_possible() const;             // mesh, options and step form allow it
     bool use_fusion(double t, double dt);     // possible and chosen (tuner or forced)
-    void advance_fused(double t, double dt);
-    void advance_enqueue(double t, double dt);  // a macro step, its CFL left in d_cfl_[0]
+    void advance_fused(double t, double dt, bool reads_cfl);
+    void advance_enqueue(double t, double dt, bool reads_cfl);  // a macro step, its CFL left in d_cfl_[0]
     void launch_fused_step(double t, double dt, const double* src, double* dst, unsigned long long* cfl_slot);
     // device time of `launches` step launches (fused: the fused step; with_fill:
     // the unfused step followed by the ghost fill) on scratch copies of q
@@ -400,7 +400,9 @@ class Context {
     // scalars
     unsigned long long* d_cfl_ = nullptr;  // [0]: advance accumulator, [1]: level / batch
     unsigned long long* h_cfl_ = nullptr;  // pinned readback of one CFL word
-    double read_cfl(const unsigned long long* d);  // copy one CFL word back and synchronize
+    bool cfl_zero_[2] = {false, false};    // words [0], [1] are zero already
+    void zero_cfl(int i, bool reads);
+    double read_cfl(int i);                // copy CFL word [i] back, zero it and synchronize
     double* d_scratch_ = nullptr;          // tagging / mass output
     size_t scratch_cap_ = 0;
     // per-patch single_step_update batching
