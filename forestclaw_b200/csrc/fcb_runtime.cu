@@ -1520,6 +1520,19 @@ void Context::launch_step_form(const StepArgs& a, int n) {
             if (!d_qalt_) arena_alloc(d_qalt_, (size_t)capacity_ * stride_ * sizeof(double));
             b.qtail = d_qalt_;
         }
+        if (opt_.solver_kind == FCB_SOLVER_ADVECTION_MANIFOLD && opt_.step_variant == 0 && !a.treg && !a.desc) {
+            // the launcher may split every patch into row bands; without memory for their
+            // source, or where the caller is recording a graph, it does not
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            cudaStreamIsCapturing(st_, &cs);
+            try {
+                if (!d_qalt_ && cs == cudaStreamCaptureStatusNone) arena_alloc(d_qalt_, (size_t)capacity_ * stride_ * sizeof(double));
+            } catch (const Error&) {
+                cudaGetLastError();
+                d_qalt_ = nullptr;
+            }
+            b.qtail = d_qalt_;
+        }
         e = launch_step(opt_.solver_kind, aux_kind_, opt_.mwaves, opt_.mx, opt_.my, opt_.mbc, b, st_,
                         opt_.claw_version);
     }

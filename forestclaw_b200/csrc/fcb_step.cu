@@ -40,6 +40,11 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* p, double 
     atomicMax(p, (unsigned long long)__double_as_longlong(v));
 }
 
+// Rows of the aux tile: a band's rows with three ahead and two behind, or all.
+__host__ __device__ constexpr int aux_rows(int ny, int nb) {
+    return nb > 1 ? ((ny - 1 + nb - 1) / nb + 5 < ny ? (ny - 1 + nb - 1) / nb + 5 : ny) : ny;
+}
+
 template <int NX, int NY, int PPB, int M, int W, int NAUX, bool PSI, int NC, bool CAPA>
 struct StepSmem {
     static constexpr int QROW = 0;
@@ -147,6 +152,11 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
     const double dtdyave = 0.5 * (dtdy + dtdy);
     SOL sol{a.grav, a.gamma, a.gamma1};
 
+    // stored aux of a launch in bands alone: the band's rows only, so more CTAs fit an SM
+    const bool few = AUXK == AUX_STORED && banded && B0 == 0;
+    const int ar0 = few ? s0 : 0;
+    const int AR = few ? aux_rows(NY, nb) : NY;
+
     // ---- aux tile ---------------------------------------------------------
     if constexpr (AUXK == AUX_SWIRL) {
         // swirl/user_4.6/b4step2.f with swirl/psi.f:
@@ -191,15 +201,16 @@ __global__ void __launch_bounds__(TPB) step_kernel(const StepArgs a) {
     } else if constexpr (AUXK == AUX_STORED) {
         if (active) {
             const double* ag = D ? D->aux : a.aux + (int64_t)slot * a.aux_stride;
+            const int re = s1 + 2 < NY ? s1 + 2 : NY;  // rows s0 .. s1 + 1 are read
             for (int k = 0; k < NAUX; ++k)
 #pragma unroll 12
-                for (int r = 0; r < NY; ++r)
-                    s_aux[((pl * NAUX + k) * NY + r) * NX + c] = ag[(k * NY + r) * NX + c];
+                for (int r = ar0; r < re; ++r)
+                    s_aux[((pl * NAUX + k) * AR + r - ar0) * NX + c] = ag[(k * NY + r) * NX + c];
         }
     }
     __syncthreads();
     auto AUXV = [&](int k, int cc, int rr) -> double {
-        if constexpr (NAUX > 0) return s_aux[((pl * NAUX + k) * NY + rr) * NX + cc];
+        if constexpr (NAUX > 0) return s_aux[((pl * NAUX + k) * AR + rr - ar0) * NX + cc];
         else return 0.0;
     };
     // Capacity: the three quotients of a cell with its kappa (dtdx1d, dtdy1d and the
@@ -688,7 +699,50 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    if (a.nbands <= 1 && a.qtail && !a.desc && !a.treg && a.npatches > 0) {
+    // shared memory of a launch in nb bands of every patch
+    auto band_bytes = [&](int nb) {
+        return (size_t)(AUXK == AUX_STORED ? L::AUX + PPB * NAUX * aux_rows(NX, nb) * NX : L::TOTAL) * sizeof(double);
+    };
+    if (AuxLayout<SOL>::CAPA && a.nbands <= 1 && a.qtail && !a.desc && !a.treg && a.npatches > 0) {
+        // Capacity: a launch of a refined mesh is 100 to 250 CTAs, bound by the latency of
+        // one sweep of NX rows (115 us for 1.5 CTAs an SM as for one).  In nb row bands
+        // it has nb times the CTAs and a band sweeps NX / nb rows and four; the nb of the
+        // least waves x rows is taken where that is a sixth less than unbanded (filament,
+        // mx = 32: 226, 155 and 128 CTAs 115 us each, in bands 82, 71 and 47 us and 5 us
+        // for the copy of the patches that the bands read).
+        static int per_wave[5] = {};
+        if (!per_wave[1]) {
+            int dev = 0, sms = 0;
+            if (cudaGetDevice(&dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+                return cudaErrorInvalidValue;
+            for (int nb = 4; nb >= 1; --nb) {
+                int occ = 0;
+                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                        &occ, step_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>, TPB, band_bytes(nb)) != cudaSuccess)
+                    return cudaErrorInvalidValue;
+                per_wave[nb] = std::max(1, sms * occ);
+            }
+        }
+        const int groups = (a.npatches + PPB - 1) / PPB;
+        auto cost = [&](int nb) {
+            return (groups * nb + per_wave[nb] - 1) / per_wave[nb] * (nb > 1 ? (NX - 1 + nb - 1) / nb + 4 : NX + 1);
+        };
+        int best = 1;
+        for (int nb = 2; nb <= 4; ++nb)
+            if (cost(nb) < cost(best)) best = nb;
+        if (best > 1 && 6 * cost(best) <= 5 * cost(1)) {
+            const int64_t vecs = (int64_t)a.npatches * (a.q_stride / 2);
+            copy_slots_kernel<<<(int)std::min<int64_t>((vecs + 255) / 256, 4096), 256, 0, st>>>(
+                a.slots, a.npatches, a.q, a.qtail, a.q_stride);
+            StepArgs t = a;
+            t.qsrc = a.qtail;
+            t.nbands = best;
+            t.band_first = 0;
+            t.qtail = nullptr;
+            return launch_one<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(t, st);
+        }
+    } else if (a.nbands <= 1 && a.qtail && !a.desc && !a.treg && a.npatches > 0) {
         // CTAs one SM array holds at once (the Roe forms: one per SM)
         static int per_wave = -1;
         if (per_wave < 0) {
@@ -723,7 +777,7 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
     if (b0 < 0 || b0 > groups) return cudaErrorInvalidValue;
     const int blocks = b0 + (groups - b0) * nb;
     if (blocks == 0) return cudaSuccess;
-    step_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM><<<blocks, TPB, bytes, st>>>(a);
+    step_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM><<<blocks, TPB, nb > 1 && b0 == 0 ? band_bytes(nb) : bytes, st>>>(a);
     return cudaGetLastError();
 }
 
