@@ -207,9 +207,10 @@ Context::Context(const fcb_options_t& o, cudaStream_t st, std::shared_ptr<Comm> 
 void Context::ensure_scalars() {
     if (d_cfl_) return;
     // [0] macro step, [1] level / batch, [2] global maximum, [3] autotuner,
-    // [4] running maximum of the asynchronous macro steps
-    check(cudaMalloc(&d_cfl_, 5 * sizeof(unsigned long long)), "cudaMalloc cfl");
-    check(cudaMemsetAsync(d_cfl_, 0, 5 * sizeof(unsigned long long), st_), "memset cfl");
+    // [4] running maximum of the asynchronous macro steps, [5] fused macro step that is
+    // waited for
+    check(cudaMalloc(&d_cfl_, 6 * sizeof(unsigned long long)), "cudaMalloc cfl");
+    check(cudaMemsetAsync(d_cfl_, 0, 6 * sizeof(unsigned long long), st_), "memset cfl");
     check(cudaHostAlloc(&h_cfl_, sizeof(unsigned long long), cudaHostAllocDefault), "cudaHostAlloc cfl");
 }
 
@@ -286,12 +287,14 @@ __global__ void cfl_publish_kernel(unsigned long long* d, volatile unsigned long
 }
 }  // namespace
 
-// Before CFL word i accumulates; `reads`: the caller reads it back itself.  A step
-// that does not may be recorded in a caller's graph, whose replays find the word as
-// the last one left it.
-void Context::zero_cfl(int i, bool reads) {
-    if (!reads || !cfl_zero_[i]) check(cudaMemsetAsync(d_cfl_ + i, 0, sizeof(unsigned long long), st_), "memset");
-    cfl_zero_[i] = false;
+// Before word i accumulates for a step whose number the call itself reads back.  Such
+// steps have words of their own (kCflLevel, kCflFused), because the host knows what
+// read_cfl left there only where nothing else writes: a step that does not wait may
+// be recorded in a caller's graph, whose replays leave their maximum in its word.
+unsigned long long* Context::zeroed_cfl(int i) {
+    if (!(cfl_zero_ >> i & 1u)) check(cudaMemsetAsync(d_cfl_ + i, 0, sizeof(unsigned long long), st_), "memset");
+    cfl_zero_ &= ~(1u << i);
+    return d_cfl_ + i;
 }
 
 // Copies CFL word i back, zeroes it and synchronizes.
@@ -300,7 +303,7 @@ double Context::read_cfl(int i) {
     check(cudaGetLastError(), "cfl");
     ++cnt_.count_kernel_launches;
     synchronize();
-    cfl_zero_[i] = true;
+    if (i != 0) cfl_zero_ |= 1u << i;
     const double c = cfl_from_bits(*h_cfl_);
     if (std::isnan(c))
         throw Error(FCB_ERR_NUMERIC, "NaN CFL: non-finite state, or a Riemann problem the reference stops on "
@@ -1552,16 +1555,14 @@ double Context::update_single_step(int level, double t, double dt) {
     if (!initialized_) throw Error(FCB_ERR_STATE, "update_single_step before initialize");
     ensure_ghosts();
     ghosts_filled_ = false;  // the step updates ghost cells; no ghost update follows
-    zero_cfl(1, true);
-    launch_level_step(level, t, dt, d_cfl_ + 1);
-    return read_cfl(1);
+    launch_level_step(level, t, dt, zeroed_cfl(kCflLevel));
+    return read_cfl(kCflLevel);
 }
 
 void Context::update_single_step_async(int level, double t, double dt) {
     if (!initialized_) throw Error(FCB_ERR_STATE, "update_single_step before initialize");
     ensure_ghosts();
     ghosts_filled_ = false;
-    cfl_zero_[0] = false;
     launch_level_step(level, t, dt, d_cfl_);
 }
 
@@ -1576,10 +1577,9 @@ double Context::single_step_update(int patchno, double t, double dt, int iter, i
     if (iter + 1 < total) return 0.0;
     d_pending_.reserve(pending_.size());
     check(cudaMemcpyAsync(d_pending_.p, pending_.data(), pending_.size() * 4, cudaMemcpyHostToDevice, st_), "pending");
-    zero_cfl(1, true);
-    launch_level_step_slots(d_pending_.p, (int)pending_.size(), t, dt, d_cfl_ + 1);
+    launch_level_step_slots(d_pending_.p, (int)pending_.size(), t, dt, zeroed_cfl(kCflLevel));
     pending_.clear();
-    return read_cfl(1);
+    return read_cfl(kCflLevel);
 }
 
 void Context::timeinterp(int level, double alpha) {
@@ -1613,7 +1613,7 @@ void Context::run_schedule(double t_curr, double dt) {
             ts[l].step_inc = 1; ts[l].dt_step = dt / rf; ts[l].total_steps = rf;
         }
     }
-    if (!dry_) zero_cfl(0, false);
+    if (!dry_) check(cudaMemsetAsync(d_cfl_, 0, sizeof(unsigned long long), st_), "memset");
     // With the step-parameter table the level updates between two ghost
     // updates (levels gmax down to some l, contiguous in the level-sorted slot
     // list) go out as one launch: they touch disjoint patches, the CFL is a
@@ -1700,8 +1700,7 @@ void Context::drop_macro_graph() {
 // later calls replay it; every call first runs the schedule "dry" on the host
 // to fill the {dt, vt} table that the step launches read.
 double Context::advance_all_levels(double t_curr, double dt) {
-    advance_enqueue(t_curr, dt, true);
-    return read_cfl(0);
+    return read_cfl(advance_enqueue(t_curr, dt, true));
 }
 
 namespace {
@@ -1728,14 +1727,13 @@ double Context::read_max_cfl() {
     return c;
 }
 
-void Context::advance_enqueue(double t_curr, double dt, bool reads_cfl) {
+int Context::advance_enqueue(double t_curr, double dt, bool reads_cfl) {
     if (!initialized_) throw Error(FCB_ERR_STATE, "advance before initialize");
     fused_used_ = 0;
     if (use_fusion(t_curr, dt)) {
         advance_fused(t_curr, dt, reads_cfl);
-        return;
+        return reads_cfl ? kCflFused : 0;
     }
-    cfl_zero_[0] = false;
     ensure_ghosts();
     // on an error, plan builds still running are joined and dropped
     struct PlanGuard {
@@ -1828,6 +1826,7 @@ void Context::advance_enqueue(double t_curr, double dt, bool reads_cfl) {
     plans_guard.armed = false;
     ++cnt_.count_amr_advance;
     ghosts_filled_ = true;  // the macro step ends with a ghost update of every level
+    return 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -2159,10 +2158,12 @@ void Context::advance_fused(double t_curr, double dt, bool reads_cfl) {
         dt_fine = dt / rf;
     }
     if (!d_qalt_) arena_alloc(d_qalt_, (size_t)capacity_ * stride_ * sizeof(double));
-    zero_cfl(0, reads_cfl);
+    unsigned long long* cfl = d_cfl_;
+    if (reads_cfl) cfl = zeroed_cfl(kCflFused);
+    else check(cudaMemsetAsync(cfl, 0, sizeof(unsigned long long), st_), "memset");
     double tk = t_curr;
     for (int k = 0; k < n_fine; ++k) {
-        launch_fused_step(tk, dt_fine, d_q_, d_qalt_, d_cfl_);
+        launch_fused_step(tk, dt_fine, d_q_, d_qalt_, cfl);
         std::swap(d_q_, d_qalt_);
         tk += dt_fine;
     }

@@ -320,7 +320,7 @@ class Context {
     bool fusion_possible() const;             // mesh, options and step form allow it
     bool use_fusion(double t, double dt);     // possible and chosen (tuner or forced)
     void advance_fused(double t, double dt, bool reads_cfl);
-    void advance_enqueue(double t, double dt, bool reads_cfl);  // a macro step, its CFL left in d_cfl_[0]
+    int advance_enqueue(double t, double dt, bool reads_cfl);  // a macro step; returns the word its CFL is in
     void launch_fused_step(double t, double dt, const double* src, double* dst, unsigned long long* cfl_slot);
     // device time of `launches` step launches (fused: the fused step; with_fill:
     // the unfused step followed by the ghost fill) on scratch copies of q
@@ -398,10 +398,11 @@ class Context {
     DevBuf<int32_t> d_groups_;
     bool ops_dirty_ = true;
     // scalars
-    unsigned long long* d_cfl_ = nullptr;  // [0]: advance accumulator, [1]: level / batch
+    static constexpr int kCflLevel = 1, kCflFused = 5;  // words of d_cfl_ that only waited-for steps use
+    unsigned long long* d_cfl_ = nullptr;  // (ensure_scalars lists the words)
     unsigned long long* h_cfl_ = nullptr;  // pinned readback of one CFL word
-    bool cfl_zero_[2] = {false, false};    // words [0], [1] are zero already
-    void zero_cfl(int i, bool reads);
+    unsigned cfl_zero_ = 0;                // bit i: word i (of those two) is zero already
+    unsigned long long* zeroed_cfl(int i);
     double read_cfl(int i);                // copy CFL word [i] back, zero it and synchronize
     double* d_scratch_ = nullptr;          // tagging / mass output
     size_t scratch_cap_ = 0;
