@@ -36,15 +36,16 @@ namespace fcb {
 
 namespace {
 
-// min(x, 0) and max(x, 0): x where its sign bit says so, else zero.
+// min(x, 0) and max(x, 0): x where its sign bit says so, else zero.  A NaN stays in one or
+// both, and so in |u|, from which the CFL number is taken (comparisons would drop it).
 __device__ __forceinline__ void split_sign(double x, double& neg, double& pos) {
     const int hi = __double2hiint(x), lo = __double2loint(x), mask = hi >> 31;
     neg = __hiloint2double(hi & mask, lo & mask);
     pos = __hiloint2double(hi & ~mask, lo & ~mask);
 }
 __device__ __forceinline__ void split_sign(float x, float& neg, float& pos) {
-    neg = dmin(x, 0.0f);
-    pos = dmax(x, 0.0f);
+    asm("min.NaN.f32 %0, %1, 0f00000000;" : "=f"(neg) : "f"(x));
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(pos) : "f"(x));
 }
 
 // A product that is rounded by itself: the mixed form's fluctuations round as those of
