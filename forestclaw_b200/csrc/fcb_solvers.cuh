@@ -1032,8 +1032,10 @@ __device__ __forceinline__ R limiter_phi(int mth, R r) {
 // times 2^400 (exact) stay in the range of the method.
 __device__ __forceinline__ double limiter_ratio(double num, double wn2, bool& ok) {
     const double r = Dv<double>(wn2 * 0x1p400, ok, 1400u).quotient(num * 0x1p400);
+    // zero, or |r| >= 2^-1000 (not rounded to a denormal) and finite (an infinite num, or
+    // one that overflows with the factor, gives a NaN here)
     const unsigned h = (unsigned)__double2hiint(r);
-    ok = ok & (h + h - 2u >= (46u << 20) - 2u);  // zero, or |r| >= 2^-1000: not rounded to a denormal
+    ok = ok & ((h + h - (46u << 20) < (4048u << 20)) | (r == 0.0));
     return r;
 }
 __device__ __forceinline__ float limiter_ratio(float num, float wn2, bool&) { return num / wn2; }

@@ -131,3 +131,17 @@ def test_operands_the_flag_refuses(check):
     assert not ok[0].any()
     out, ok = check(np.array([0.0, -0.0]), np.array([3.0, 3.0]))
     assert ok[0].all() and (out[0] == 0).all()
+
+
+def test_dividends_the_flag_refuses(check):
+    """Infinite, NaN and huge dividends: the operator's infinity, not the residual's NaN."""
+    a = np.array([np.inf, -np.inf, np.nan, 1e300, -1e300, 1.7e308, 2.0 ** 123])
+    for b in (1.0, 1e-250, 3.0):
+        _, ok = check(a, np.full_like(a, b))
+        assert not ok[0].any()
+    a = np.array([np.nextafter(2.0 ** 123, 0), -1e37, 2.0 ** -960, -(2.0 ** -960)])
+    for b in (2.0 ** -900, 0.7, 2.0 ** 59 * 1.3):
+        out, ok = check(a, np.full_like(a, b))
+        assert ok[0].all()
+        big = np.abs(out[1]) >= 2.0 ** -1022
+        assert np.isfinite(out[1]).all() and np.array_equal(out[0][big], out[1][big])
