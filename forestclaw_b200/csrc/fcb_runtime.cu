@@ -1843,6 +1843,9 @@ std::map<std::vector<int>, int> g_step_form_cache, g_ghost_unroll_cache;
 
 int default_step_form(const fcb_options_t& o) {
     if (o.solver_kind == SOLVER_ADVECTION_MANIFOLD) return 1;  // capacity: four-barrier form only
+    // scalar advection has a pipelined form of patches up to mx = 32; the larger ones that
+    // are tuned at all (FP64, clawpack 4.6) run the four-barrier form
+    if (o.solver_kind == SOLVER_ADVECTION && o.mx > 32) return 1;
     return 3;
 }
 }  // namespace
