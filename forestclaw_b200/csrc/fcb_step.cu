@@ -28,6 +28,7 @@
 #include <cstdio>
 
 #include "fcb_device.h"
+#include "fcb_launch.hpp"
 #include "fcb_solvers.cuh"
 
 namespace fcb {
@@ -692,17 +693,23 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
     static_assert(PPB >= 1, "patch wider than the CTA");
     using L = StepSmem<NX, NX, PPB, SOL::M, SOL::W, NAUX, AUXK == AUX_SWIRL, SOL::NC, AuxLayout<SOL>::CAPA>;
     const size_t bytes = (size_t)L::TOTAL * sizeof(double);
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(step_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    constexpr auto kernel = step_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>;
     // shared memory of a launch in nb bands of every patch
     auto band_bytes = [&](int nb) {
         return (size_t)(AUXK == AUX_STORED ? L::AUX + PPB * NAUX * aux_rows(NX, nb) * NX : L::TOTAL) * sizeof(double);
     };
+    // CTAs one SM array holds at once of a launch in nb bands, at [nb - 1] (the Roe forms:
+    // one per SM)
+    constexpr int NB = AuxLayout<SOL>::CAPA ? 4 : 1;
+    static PerDevice<NB> kept;
+    int per_wave[NB];
+    const cudaError_t e = per_device(kept, per_wave, [&](int* n) {
+        cudaError_t f = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        for (int nb = 1; nb <= NB && f == cudaSuccess; ++nb)
+            f = resident_ctas(kernel, TPB, nb > 1 ? band_bytes(nb) : bytes, n + nb - 1);
+        return f;
+    });
+    if (e != cudaSuccess) return e;
     if (AuxLayout<SOL>::CAPA && a.nbands <= 1 && a.qtail && !a.desc && !a.treg && a.npatches > 0) {
         // Capacity: a launch of a refined mesh is 100 to 250 CTAs, bound by the latency of
         // one sweep of NX rows (115 us for 1.5 CTAs an SM as for one).  In nb row bands
@@ -710,23 +717,10 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
         // least waves x rows is taken where that is a sixth less than unbanded (filament,
         // mx = 32: 226, 155 and 128 CTAs 115 us each, in bands 82, 71 and 47 us and 5 us
         // for the copy of the patches that the bands read).
-        static int per_wave[5] = {};
-        if (!per_wave[1]) {
-            int dev = 0, sms = 0;
-            if (cudaGetDevice(&dev) != cudaSuccess ||
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-                return cudaErrorInvalidValue;
-            for (int nb = 4; nb >= 1; --nb) {
-                int occ = 0;
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                        &occ, step_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>, TPB, band_bytes(nb)) != cudaSuccess)
-                    return cudaErrorInvalidValue;
-                per_wave[nb] = std::max(1, sms * occ);
-            }
-        }
         const int groups = (a.npatches + PPB - 1) / PPB;
         auto cost = [&](int nb) {
-            return (groups * nb + per_wave[nb] - 1) / per_wave[nb] * (nb > 1 ? (NX - 1 + nb - 1) / nb + 4 : NX + 1);
+            const int w = per_wave[std::min(nb, NB) - 1];
+            return (groups * nb + w - 1) / w * (nb > 1 ? (NX - 1 + nb - 1) / nb + 4 : NX + 1);
         };
         int best = 1;
         for (int nb = 2; nb <= 4; ++nb)
@@ -743,19 +737,8 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
             return launch_one<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(t, st);
         }
     } else if (a.nbands <= 1 && a.qtail && !a.desc && !a.treg && a.npatches > 0) {
-        // CTAs one SM array holds at once (the Roe forms: one per SM)
-        static int per_wave = -1;
-        if (per_wave < 0) {
-            int dev = 0, sms = 0, occ = 0;
-            if (cudaGetDevice(&dev) != cudaSuccess ||
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, step_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>,
-                                                              TPB, bytes) != cudaSuccess)
-                return cudaErrorInvalidValue;
-            per_wave = sms * occ;
-        }
         int tb = 1;
-        const int b0 = tail_plan((a.npatches + PPB - 1) / PPB, per_wave, &tb);
+        const int b0 = tail_plan((a.npatches + PPB - 1) / PPB, per_wave[0], &tb);
         if (b0 >= 0) {
             const int first = b0 * PPB, ntail = a.npatches - first;
             const int64_t vecs = (int64_t)ntail * (a.q_stride / 2);
@@ -777,7 +760,7 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
     if (b0 < 0 || b0 > groups) return cudaErrorInvalidValue;
     const int blocks = b0 + (groups - b0) * nb;
     if (blocks == 0) return cudaSuccess;
-    step_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM><<<blocks, TPB, nb > 1 && b0 == 0 ? band_bytes(nb) : bytes, st>>>(a);
+    kernel<<<blocks, TPB, nb > 1 && b0 == 0 ? band_bytes(nb) : bytes, st>>>(a);
     return cudaGetLastError();
 }
 

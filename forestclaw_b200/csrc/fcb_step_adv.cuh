@@ -26,9 +26,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 
 #include "fcb_device.h"
+#include "fcb_launch.hpp"
 #include "fcb_solvers.cuh"
 #include "fcb_strip.cuh"
 
@@ -353,18 +353,15 @@ template <typename R, int AUXK, int TPB, int LIM>
 cudaError_t launch_adv_one(const StepArgs& a, cudaStream_t st) {
     using L = AdvSmem<TPB, R>;
     constexpr auto kernel = step_kernel_adv<R, AUXK, TPB, LIM>;
-    static std::atomic<int> per_wave{0};
-    if (per_wave.load() == 0) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::bytes(kStripRowsMax));
-        if (e != cudaSuccess) return e;
-        int dev = 0, sms = 0, occ = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, TPB, L::bytes(256))) != cudaSuccess) return e;
-        per_wave.store(std::max(1, sms * occ));
-    }
+    static PerDevice<> kept;
+    int per_wave = 0;
+    const cudaError_t e = per_device(kept, &per_wave, [&](int* n) {
+        const cudaError_t f = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::bytes(kStripRowsMax));
+        return f != cudaSuccess ? f : resident_ctas(kernel, TPB, L::bytes(256), n);
+    });
+    if (e != cudaSuccess) return e;
     StepArgs b = a;
-    strip_plan(b.strip, TPB - 4, per_wave.load(), 5);
+    strip_plan(b.strip, TPB - 4, per_wave, 5);
     kernel<<<b.strip.nsx * b.strip.nsy, TPB, L::bytes(b.strip.h), st>>>(b);
     return cudaGetLastError();
 }

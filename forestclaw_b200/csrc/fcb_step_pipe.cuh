@@ -39,6 +39,7 @@
 #include <type_traits>
 
 #include "fcb_device.h"
+#include "fcb_launch.hpp"
 #include "fcb_solvers.cuh"
 
 namespace fcb {
@@ -757,12 +758,13 @@ cudaError_t launch_pipe_one(const StepArgs& a, cudaStream_t st) {
     using L = PipeSmem<NX, PPB, SOL::M, SOL::W, NAUX, AUXK == AUX_SWIRL, typename SOL::Real>;
     const size_t bytes = (size_t)L::BYTES;
     constexpr auto kernel = pipe_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>();
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    static PerDevice<> kept;
+    int none;
+    const cudaError_t e = per_device(kept, &none, [&](int* n) {
+        *n = 0;
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
+    if (e != cudaSuccess) return e;
     const int blocks = (a.npatches + PPB - 1) / PPB;
     if (blocks == 0) return cudaSuccess;
     kernel<<<blocks, TPB, bytes, st>>>(a);

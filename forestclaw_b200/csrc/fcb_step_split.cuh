@@ -39,10 +39,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <type_traits>
 
 #include "fcb_device.h"
+#include "fcb_launch.hpp"
 #include "fcb_solvers.cuh"
 #include "fcb_strip.cuh"
 
@@ -878,24 +878,21 @@ cudaError_t launch_split_one(const StepArgs& a, cudaStream_t st) {
     using L = SplitSmem<SOL, PPB * NXC, NAUX>;
     static_assert(L::BYTES <= 227 * 1024, "shared memory of the CTA");
     constexpr auto kernel = step_kernel_split<SOL, MXP, NAUX, HALF, LIM, TSYNC>;
-    static std::atomic<int> per_wave{0};  // CTAs the SM array holds at once (the same on every launch)
-    if (per_wave.load() == 0) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES);
-        if (e != cudaSuccess) return e;
-        int dev = 0, sms = 0, occ = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 2 * HALF, L::BYTES)) != cudaSuccess) return e;
-        per_wave.store(std::max(1, sms * occ));
-    }
     if (a.npatches <= 0) return cudaSuccess;
+    static PerDevice<> kept;
+    int per_wave = 0;  // CTAs the SM array holds at once
+    const cudaError_t e = per_device(kept, &per_wave, [&](int* n) {
+        const cudaError_t f = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES);
+        return f != cudaSuccess ? f : resident_ctas(kernel, 2 * HALF, L::BYTES, n);
+    });
+    if (e != cudaSuccess) return e;
     StepArgs b = a;
     int blocks;
     if constexpr (MXP == 0) {
-        strip_plan(b.strip, HALF - 4, per_wave.load(), 7);
+        strip_plan(b.strip, HALF - 4, per_wave, 7);
         blocks = b.strip.nsx * b.strip.nsy;
     } else {
-        b.ppc = split_patches_per_cta(a.npatches, PPB, per_wave.load());
+        b.ppc = split_patches_per_cta(a.npatches, PPB, per_wave);
         blocks = (a.npatches + b.ppc - 1) / b.ppc;
     }
     kernel<<<blocks, 2 * HALF, L::BYTES, st>>>(b);
