@@ -112,6 +112,14 @@ __device__ __forceinline__ void copy_async8(double* dst, const double* src) {
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// The barrier of a row.  The two halves of the CTA meet at it from different places, which
+// __syncthreads() is not made for (one call, reached by the whole CTA); a barrier with its
+// number and count of threads is.  Both halves pass it NY + 3 times.
+template <int THREADS>
+__device__ __forceinline__ void row_barrier() {
+    asm volatile("barrier.sync 1, %0;" ::"n"(THREADS) : "memory");
+}
+
 // The time-sync registers are accumulated for the shallow-water Roe solver in
 // FP64, the one whose conservative flux the flux store has.
 template <class SOL>
@@ -538,7 +546,7 @@ __global__ void __launch_bounds__(2 * HALF) step_kernel_split(const StepArgs a) 
                 }
             }
             if constexpr (ASYNC) neg = neg1;
-            __syncthreads();
+            row_barrier<2 * HALF>();
             const int n0 = a2;
             a2 = a1;
             a1 = a0;
@@ -825,7 +833,7 @@ __global__ void __launch_bounds__(2 * HALF) step_kernel_split(const StepArgs a) 
                     }
                 }
             }
-            __syncthreads();
+            row_barrier<2 * HALF>();
             const int n0 = a2;
             a2 = a1;
             a1 = a0;
