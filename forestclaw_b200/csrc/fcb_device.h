@@ -41,6 +41,7 @@ struct StripArgs {
     int32_t n, lg, lgp, nxp;  // nxp: columns of a patch with its ghost columns
     int32_t bc[4];        // mthbc of the domain's sides (left, right, bottom, top), 0: periodic
     double ax, ay;        // lower-left corner of the domain
+    int32_t patches;      // 1: cell sizes differ by patch, so patches are swept one by one
     int32_t w, h, nsx, nsy;  // set by the launcher
 };
 

@@ -2053,7 +2053,9 @@ void Context::build_strip_grid() {
     for (int k = 0; k < 4; ++k) strip_.bc[k] = (k < 2 ? opt_.periodic_x : opt_.periodic_y) ? 0 : opt_.mthbc[k];
     // a strip takes every cell size and position from the domain's corner and one
     // spacing: the patches' own must be the same numbers, which they are when the
-    // cell edges and centres are exact in double precision
+    // cell edges and centres are exact in double precision.  Where they are not, scalar
+    // advection is fused patch by patch (fcb_step_pipe.cuh); the systems' patches with their
+    // ghost fill (fcb_step_split.cuh) are faster than such a form of them was.
     const double dx = h_meta_[slot_of_[0]].dx, dy = h_meta_[slot_of_[0]].dy;
     auto exact = [&](double lo, double hi, double d) {
         int e;
@@ -2065,18 +2067,19 @@ void Context::build_strip_grid() {
         return std::fmod(lo, unit) == 0.0 &&
                std::max(std::fabs(lo), std::fabs(hi)) + 4.0 * d <= std::ldexp(unit, 53);
     };
-    if (!exact(opt_.ax, opt_.bx, dx) || !exact(opt_.ay, opt_.by, dy)) return;
+    bool strips = exact(opt_.ax, opt_.bx, dx) && exact(opt_.ay, opt_.by, dy);
     std::vector<int32_t> grid((size_t)P * P, -1);
     const int sh = QuadForest::kMaxLevel - gmax_;
     for (int p = 0; p < num_patches(); ++p) {
         const Leaf& l = forest_.leaves[p];
         const PatchMeta& m = h_meta_[slot_of_[p]];
         const int px = l.x >> sh, py = l.y >> sh;
-        if (m.dx != dx || m.dy != dy || m.xlower != opt_.ax + (double)(px * opt_.mx) * dx ||
-            m.ylower != opt_.ay + (double)(py * opt_.my) * dy)
-            return;
+        strips = strips && m.dx == dx && m.dy == dy && m.xlower == opt_.ax + (double)(px * opt_.mx) * dx &&
+                 m.ylower == opt_.ay + (double)(py * opt_.my) * dy;
         grid[(size_t)py * P + px] = slot_of_[p];
     }
+    if (!strips && (opt_.solver_kind != FCB_SOLVER_ADVECTION || opt_.mx > 32)) return;
+    strip_.patches = strips ? 0 : 1;
     d_grid_.reserve(grid.size());
     check(cudaMemcpy(d_grid_.p, grid.data(), grid.size() * sizeof(int32_t), cudaMemcpyHostToDevice), "strip grid");
     strip_.grid = d_grid_.p;
@@ -2107,7 +2110,7 @@ bool Context::use_fusion(double t, double dt) {
     int nb = 0;
     while ((1 << (nb + 1)) <= own_count_) ++nb;
     const std::vector<int> key = {opt_.solver_kind, aux_kind_, opt_.mwaves, opt_.mx, opt_.claw_version, opt_.precision,
-                                  fixed_lim ? opt_.mthlim[0] : -1, nb};
+                                  fixed_lim ? opt_.mthlim[0] : -1, nb, strip_.patches};
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_fusion_cache.find(key);

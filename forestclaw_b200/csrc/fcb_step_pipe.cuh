@@ -27,7 +27,12 @@
 //   q = q - dtdx*(fm(i+1,j) - fp(i,j)) - dtdy*(gm(i,j+1) - gp(i,j)).
 // It serves scalar advection on meshes of several levels, served and partitioned
 // solves and level calls; the systems run fcb_step_split.cuh, meshes of one level
-// fcb_step_adv.cuh.
+// fcb_step_adv.cuh.  FUSED: a mesh of one level whose cell edges are not exact in double
+// precision (an extent like 0 to 0.3).  Its patches differ in dx by a rounding, so strips
+// that cross them would not give each patch's own numbers; the patches are swept one by
+// one, their ghost cells read from the neighbours' interiors (fcb_strip.cuh).  B200,
+// mx = 16, us a step, unfused with its ghost fill -> fused: FP64 16,384 patches 149 -> 131,
+// 65,536 558 -> 500; mixed 136 -> 112, 475 -> 387.
 // The kernel is a template on the compute type R of the Riemann solves,
 // limiters and transverse parts (SOL::Real): R = double is the FP64 form,
 // compiled without FMA contraction (fcb_step_pipe.cu); R = float is the mixed
@@ -41,6 +46,7 @@
 #include "fcb_device.h"
 #include "fcb_launch.hpp"
 #include "fcb_solvers.cuh"
+#include "fcb_strip.cuh"
 
 namespace fcb {
 
@@ -112,9 +118,8 @@ struct PipeState {
     static constexpr int W = SOL::W;
     double qcur[M], q_m1[M];                             // q(c, s), q(c, s-1)
     double qpre[M];                                      // q(c, s+1), loaded one iteration ahead
-    // scalar case: q(c, s-2..s-4) kept from their loads, so the update of row
+    // q(c, s-2..s-4) kept from their loads, so the update of row
     // s-4 reads its old value from registers instead of memory
-    static constexpr bool DELAY = M == 1;
     double q_m2[M], q_m3[M], q_m4[M];
     R yw_f[W][M], ys_f[W], yam_f[M], yap_f[M], ydotl[W];  // raw y-interface s-1
     typename SOL::Roe yR_f;
@@ -131,7 +136,7 @@ struct PipeState {
 // Per-thread constants: column, flags and this thread's element of the rings.
 template <typename R>
 struct PipeThread {
-    double* q;        // q of the patch, offset to column c
+    double* q;        // q of the patch, offset to column c (FUSED: see fused_row)
     double* qlast;    // qlast of the patch, offset to column c
     const double* aux;
     R* rb;            // this thread's element of the R rings
@@ -144,13 +149,30 @@ struct PipeThread {
     bool active, save_last, ycol, node;
 };
 
+template <int NX, bool SWIRL>
+__host__ __device__ constexpr int pipe_threads_per_patch() { return SWIRL ? NX + 1 : NX; }
+
 // ring slot of row s - d when s == J (mod D) is known at compile time
 __host__ __device__ constexpr int cslot(int J, int d, int D) { return ((J - d) % D + D) % D; }
+
+// FUSED: where row `row` of column c of the patch at place `at` of the mesh has its value
+// (a wall mirrors a scalar without a sign).  The interior rows of a column follow one
+// another in one patch: T.q is their base, and in a column that is written the base in
+// the arena written is as far from it as the arenas are.  (With a pointer of its own for
+// the rows read the mixed form spills: 422 us a step of 65,536 patches, 382 so.)
+template <int MX, int MBC>
+__device__ __forceinline__ const double* fused_row(const StepArgs& a, int at, int c, int row) {
+    const StripArgs& g = a.strip;
+    bool wall;
+    const int x = strip_inside((at & ((1 << g.lgp) - 1)) * MX + c - MBC, g.n, g.bc[0], g.bc[1], wall);
+    const int y = strip_inside((at >> g.lgp) * MX + row - MBC, g.n, g.bc[2], g.bc[3], wall);
+    return a.qsrc + ((int64_t)strip_slot(g, x, y) * a.q_stride + strip_cell(g, x, y));
+}
 
 // One row-iteration.  J >= 0: s == J (mod 4) at compile time, so every ring
 // slot is a constant; STEADY: s in [4, NY-2], where every stage is active for
 // every row and the row-range tests vanish.
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int PPB, int LIM, int J, bool STEADY>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int PPB, int LIM, bool FUSED, int J, bool STEADY>
 __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                                           const PipeThread<typename SOL::Real>& T, PipeState<SOL>& S, int s) {
     using R = typename SOL::Real;
@@ -177,7 +199,7 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
 
     // prefetch q(c, s+2); the old value of q(c, s-4) for this iteration's update
     double qnext[M], qold[M];
-    const bool upd = T.active && (V5 ? (s - 4 >= MBC && s - 4 <= MBC + MX - 1 && c >= MBC && c <= MBC + MX - 1)
+    const bool upd = T.active && (V5 || FUSED ? (s - 4 >= MBC && s - 4 <= MBC + MX - 1 && c >= MBC && c <= MBC + MX - 1)
                                      : ((STEADY || (s - 4 >= 0 && s - 4 <= NY - 2)) && c <= NX - 2));
     {
         // prefetch two rows ahead; the last steady iteration (s = 4 + 4*((NY-5)/4) - 1)
@@ -186,9 +208,18 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
         const bool on = T.active && ((STEADY && STEADY_IN) || s + 2 < NY);
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            qnext[m] = on ? T.q[((int64_t)m * NY + s + 2) * NX] : 0.0;
-            if constexpr (PipeState<SOL>::DELAY) qold[m] = S.q_m4[m];
-            else qold[m] = upd ? T.q[((int64_t)m * NY + s - 4) * NX] : 0.0;
+            static_assert(M == 1, "scalar equations");
+            const double* from = T.q + (s + 2) * NX;
+            if constexpr (FUSED) {
+                // two rows after the interior; the place is found again, not kept in a register
+                if (J < 2 && s + 2 >= MBC + MX && on) {
+                    unsigned t;
+                    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+                    from = fused_row<MX, MBC>(a, blockIdx.x * PPB + t / pipe_threads_per_patch<NX, SWIRL>(), c, s + 2);
+                }
+            }
+            qnext[m] = on ? *from : 0.0;
+            qold[m] = S.q_m4[m];
         }
     }
 
@@ -233,7 +264,11 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
                 const double fpv = (fxp0 + gyu_l) + gyd;   // fp(i, j)
                 const double gmv = GXs_new[m] + (double)S.FYm2[m];    // gm(i, j+1)
                 const double gpv = S.GXs_prev[m] + (double)S.FYp3[m];  // gp(i, j)
-                T.q[((int64_t)m * NY + r) * NX] = qold[m] - T.dtdx * (fmv - fpv) - T.dtdy * (gmv - gpv);
+                double* to = T.q + r * NX;
+                if constexpr (FUSED)
+                    to = reinterpret_cast<double*>(reinterpret_cast<char*>(to) +
+                                                   (reinterpret_cast<char*>(a.q) - reinterpret_cast<const char*>(a.qsrc)));
+                *to = qold[m] - T.dtdx * (fmv - fpv) - T.dtdy * (gmv - gpv);
             }
         }
 #pragma unroll
@@ -526,11 +561,9 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
         for (int m = 0; m < M; ++m) {
             S.yam_f[m] = yam_n[m];
             S.yap_f[m] = yap_n[m];
-            if constexpr (PipeState<SOL>::DELAY) {
-                S.q_m4[m] = S.q_m3[m];
-                S.q_m3[m] = S.q_m2[m];
-                S.q_m2[m] = S.q_m1[m];
-            }
+            S.q_m4[m] = S.q_m3[m];
+            S.q_m3[m] = S.q_m2[m];
+            S.q_m2[m] = S.q_m1[m];
             S.q_m1[m] = S.qcur[m];
             S.qcur[m] = S.qpre[m];
             S.qpre[m] = qnext[m];
@@ -561,9 +594,6 @@ __device__ __forceinline__ void pipe_iter(const StepArgs& a, const SOL& sol,
     __syncthreads();
 }
 
-template <int NX, bool SWIRL>
-__host__ __device__ constexpr int pipe_threads_per_patch() { return SWIRL ? NX + 1 : NX; }
-
 }  // namespace
 
 // The mixed scalar form runs with the register budget cut for six resident
@@ -577,7 +607,7 @@ constexpr bool pipe_six_ctas() {
     return sizeof(typename SOL::Real) == 4 && SOL::M == 1;
 }
 
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
 __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     constexpr int M = SOL::M;
     constexpr int W = SOL::W;
@@ -604,7 +634,7 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     const int pls = patch_ok ? pl : 0;  // threads without a patch read (never write) patch 0's rows
     const int cc = c < NX ? c : NX - 1;
     const PatchDesc* D = (a.desc && patch_ok) ? a.desc + pg : nullptr;  // mixed-solve launch
-    const int slot = (patch_ok && !a.desc) ? a.slots[pg] : 0;
+    const int slot = (patch_ok && !a.desc) ? (FUSED ? a.strip.grid[pg] : a.slots[pg]) : 0;
     const PatchMeta meta = D ? D->meta : (patch_ok ? a.meta[slot] : PatchMeta{0, 0, 1, 1, 0, 0});
     const int req = D ? D->req : -1;
     SOL sol{R(a.grav), R(a.gamma), R(a.gamma1), R(a.drytol)};
@@ -616,6 +646,7 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     T.save_last = active && (meta.flags & PATCH_SAVE_LAST);
     T.ycol = active && c >= 1 && c <= NX - 2;
     T.q = (D ? D->q : a.q + (int64_t)slot * a.q_stride) + cc;
+    if constexpr (FUSED) T.q = const_cast<double*>(active ? fused_row<MX, MBC>(a, pg, cc, MBC) : a.qsrc) - MBC * NX;
     T.qlast = (D ? D->qlast : a.qlast + (int64_t)slot * a.q_stride) + cc;
     T.aux = (AUXK == AUX_STORED && active) ? (D ? D->aux : a.aux + (int64_t)slot * a.aux_stride) + cc : nullptr;
     T.rb = rsm + pls * NX + cc;
@@ -637,8 +668,8 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     PipeState<SOL> S;
 #pragma unroll
     for (int m = 0; m < M; ++m) {
-        S.qcur[m] = active ? T.q[(int64_t)m * NY * NX] : 0.0;
-        S.qpre[m] = active ? T.q[((int64_t)m * NY + 1) * NX] : 0.0;
+        S.qcur[m] = active ? (FUSED ? *fused_row<MX, MBC>(a, pg, cc, 0) : T.q[0]) : 0.0;
+        S.qpre[m] = active ? (FUSED ? *fused_row<MX, MBC>(a, pg, cc, 1) : T.q[NX]) : 0.0;
         S.q_m1[m] = 0.0;
         S.q_m2[m] = S.q_m3[m] = S.q_m4[m] = 0.0;
         S.yam_f[m] = S.yap_f[m] = R(0);
@@ -697,15 +728,15 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
 
     // ---- rows: ramp-up, steady state (unrolled by the ring period 4), ramp-down ----
     int s = 0;
-    for (; s < 4; ++s) pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, -1, false>(a, sol, T, S, s);
+    for (; s < 4; ++s) pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, FUSED, -1, false>(a, sol, T, S, s);
     constexpr int NSTEADY = NY - 5;  // s = 4 .. NY-2
     for (int rnd = 0; rnd < NSTEADY / 4; ++rnd, s += 4) {
-        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 0, true>(a, sol, T, S, s);
-        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 1, true>(a, sol, T, S, s + 1);
-        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 2, true>(a, sol, T, S, s + 2);
-        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, 3, true>(a, sol, T, S, s + 3);
+        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, FUSED, 0, true>(a, sol, T, S, s);
+        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, FUSED, 1, true>(a, sol, T, S, s + 1);
+        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, FUSED, 2, true>(a, sol, T, S, s + 2);
+        pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, FUSED, 3, true>(a, sol, T, S, s + 3);
     }
-    for (; s <= NY + 2; ++s) pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, -1, false>(a, sol, T, S, s);
+    for (; s <= NY + 2; ++s) pipe_iter<SOL, MX, MBC, AUXK, NAUX, PPB, LIM, FUSED, -1, false>(a, sol, T, S, s);
 
     // ---- CFL: warp max, one atomic per warp ----
     // flux2: cfl = max(cfl, dtdx*s, -dtdx*s) over the interfaces.  Rounding is
@@ -728,21 +759,30 @@ __device__ __forceinline__ void step_pipe_body(const StepArgs& a) {
     }
 }
 
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
 __global__ void __launch_bounds__(TPB) step_kernel_pipe(const StepArgs a) {
-    step_pipe_body<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(a);
+    step_pipe_body<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>(a);
 }
 
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
 __global__ void __launch_bounds__(TPB, 6) step_kernel_pipe_six(const StepArgs a) {
-    step_pipe_body<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(a);
+    step_pipe_body<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>(a);
 }
 
-// the one kernel of the two that a form uses (only that one is instantiated)
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
+// the FP64 form of patches with the ghost exchange folded in: left to the compiler the
+// swirl velocities take 142 registers and three CTAs fit an SM (570 us a step of 65,536
+// patches of mx = 16, 494 so)
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
+__global__ void __launch_bounds__(TPB, 4) step_kernel_pipe_four(const StepArgs a) {
+    step_pipe_body<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>(a);
+}
+
+// the one kernel of the three that a form uses (only that one is instantiated)
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED>
 constexpr auto pipe_kernel() {
-    if constexpr (pipe_six_ctas<SOL>()) return step_kernel_pipe_six<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>;
-    else return step_kernel_pipe<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>;
+    if constexpr (pipe_six_ctas<SOL>()) return step_kernel_pipe_six<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>;
+    else if constexpr (FUSED) return step_kernel_pipe_four<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>;
+    else return step_kernel_pipe<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>;
 }
 
 // ---------------------------------------------------------------------------
@@ -750,14 +790,16 @@ constexpr auto pipe_kernel() {
 // ---------------------------------------------------------------------------
 namespace {
 
-template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
+template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM, bool FUSED = false>
 cudaError_t launch_pipe_one(const StepArgs& a, cudaStream_t st) {
+    if constexpr (!FUSED)
+        if (a.strip.grid) return launch_pipe_one<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, true>(a, st);
     constexpr int NX = MX + 2 * MBC;
     constexpr int PPB = TPB / pipe_threads_per_patch<NX, AUXK == AUX_SWIRL>();
     static_assert(PPB >= 1, "patch wider than the CTA");
     using L = PipeSmem<NX, PPB, SOL::M, SOL::W, NAUX, AUXK == AUX_SWIRL, typename SOL::Real>;
     const size_t bytes = (size_t)L::BYTES;
-    constexpr auto kernel = pipe_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>();
+    constexpr auto kernel = pipe_kernel<SOL, MX, MBC, AUXK, NAUX, TPB, LIM, FUSED>();
     static PerDevice<> kept;
     int none;
     const cudaError_t e = per_device(kept, &none, [&](int* n) {
@@ -813,7 +855,7 @@ cudaError_t launch_step_pipe_v(int solver, int aux_kind, int mwaves, int mx, int
     switch (solver) {
         case SOLVER_ADVECTION:
             if (mwaves != 1) return cudaErrorNotSupported;
-            if (a.strip.grid) {
+            if (a.strip.grid && !a.strip.patches) {
                 if constexpr (std::is_same_v<R, float>) return launch_step_adv_mixed(aux_kind, V5 ? 5 : 4, a, st);
                 else return launch_step_adv(aux_kind, V5 ? 5 : 4, a, st);
             }

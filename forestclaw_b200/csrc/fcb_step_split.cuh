@@ -938,6 +938,7 @@ cudaError_t launch_split_ts(const StepArgs& a, cudaStream_t st) {
 
 template <class SOL, int NAUX>
 cudaError_t launch_split_mx(int mx, const StepArgs& a, cudaStream_t st) {
+    if (a.strip.grid && a.strip.patches) return cudaErrorNotSupported;
     if (a.strip.grid) return launch_split_ts<SOL, 0, NAUX>(a, st);  // strips take patches of any size
     switch (mx) {
         case 8: return launch_split_ts<SOL, 8, NAUX>(a, st);
