@@ -865,13 +865,14 @@ Context::PlanWork& Context::plan_work(size_t k) {
     return *plan_work_[k];
 }
 
-// Keeps at most 64 MB of build memory (meshes of about 20,000 patches).
+// The contexts of a process keep at most 64 MB of build memory together (that of meshes
+// of about 20,000 patches).
+std::atomic<size_t> Context::plan_bytes_{0};
+
 void Context::trim_plan_work() {
-    size_t kept = 0;
-    for (auto& w : plan_work_) {
-        kept += w->bytes();
-        if (kept > ((size_t)64 << 20)) *w = PlanWork{};
-    }
+    plan_kept_.clear();
+    for (auto& w : plan_work_)
+        if (!plan_kept_.add(w->bytes())) *w = PlanWork{};
 }
 
 const GhostPlan& Context::commit_plan(const std::tuple<int, int, int>& key, PlanBuild& b) {

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <map>
 #include <stdexcept>
@@ -14,6 +15,7 @@
 #include <memory>
 
 #include "../../include/fclaw_b200.h"
+#include "fcb_budget.hpp"
 #include "fcb_comm.hpp"
 #include "fcb_device.h"
 #include "fcb_forest.hpp"
@@ -278,6 +280,8 @@ class Context {
     size_t h_ts_groups_pinned_cap_ = 0;
     std::vector<std::tuple<int, int, int>> plan_todo_;
     std::vector<std::unique_ptr<PlanWork>> plan_work_;  // one per build that runs at once
+    static std::atomic<size_t> plan_bytes_;  // kept by all contexts
+    KeptBytes plan_kept_{plan_bytes_, (size_t)64 << 20};
     std::vector<std::exception_ptr> plan_err_;
     std::vector<std::thread> plan_threads_;
     // pinned staging of the op and group buffers, and the event of its last upload
