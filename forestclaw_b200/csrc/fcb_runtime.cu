@@ -356,6 +356,11 @@ void Context::ensure_capacity(int n) {
         }
         p = np;
     };
+    // the scratch arena (fused steps, row bands: reallocated at its next use) first: its
+    // memory serves the new arenas
+    arena_free(d_qalt_);
+    d_qalt_ = nullptr;
+    no_band_room_ = false;
     grow(d_q_);
     grow(d_qlast_);
     grow(d_qti_);
@@ -373,8 +378,6 @@ void Context::ensure_capacity(int n) {
         d_treg_ = np;
     }
     if (!opt_.use_fixed_dt) grow(d_qsave_);
-    arena_free(d_qalt_);  // the second arena of fused steps: reallocated at its next use
-    d_qalt_ = nullptr;
     if (aux_kind_ == AUX_STORED) {  // recomputed for every patch by mesh_changed
         arena_free(d_aux_);
         d_aux_ = nullptr;
@@ -1526,14 +1529,18 @@ void Context::launch_step_form(const StepArgs& a, int n) {
         }
         if (opt_.solver_kind == FCB_SOLVER_ADVECTION_MANIFOLD && opt_.step_variant == 0 && !a.treg && !a.desc) {
             // the launcher may split every patch into row bands; without memory for their
-            // source, or where the caller is recording a graph, it does not
+            // source (asked for once per arena size), or where the caller is recording a
+            // graph, it does not
             cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
             cudaStreamIsCapturing(st_, &cs);
-            try {
-                if (!d_qalt_ && cs == cudaStreamCaptureStatusNone) arena_alloc(d_qalt_, (size_t)capacity_ * stride_ * sizeof(double));
-            } catch (const Error&) {
-                cudaGetLastError();
-                d_qalt_ = nullptr;
+            if (!d_qalt_ && !no_band_room_ && cs == cudaStreamCaptureStatusNone) {
+                try {
+                    arena_alloc(d_qalt_, (size_t)capacity_ * stride_ * sizeof(double));
+                } catch (const Error&) {
+                    cudaGetLastError();
+                    d_qalt_ = nullptr;
+                    no_band_room_ = true;
+                }
             }
             b.qtail = d_qalt_;
         }

@@ -336,6 +336,7 @@ class Context {
     void ensure_ghosts();  // run the deferred ghost update, if one is pending
   private:
     double* d_qalt_ = nullptr;
+    bool no_band_room_ = false;   // no memory for d_qalt_ as the source of row bands
     DevBuf<int32_t> d_grid_;      // slots of a mesh of one level by place
     StripArgs strip_{};           // grid null: the mesh has no strips
     bool ghosts_stale_ = false;
