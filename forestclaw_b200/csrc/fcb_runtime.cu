@@ -1544,8 +1544,11 @@ void Context::launch_step_form(const StepArgs& a, int n) {
             }
             b.qtail = d_qalt_;
         }
+        int bands = 1;
         e = launch_step(opt_.solver_kind, aux_kind_, opt_.mwaves, opt_.mx, opt_.my, opt_.mbc, b, st_,
-                        opt_.claw_version);
+                        opt_.claw_version, &bands);
+        if (bands > 1) ++cnt_.count_kernel_launches;  // the copy that the bands read
+        bands_used_ = bands;
     }
     check(e, "step");
     cnt_.count_single_step += n;

@@ -687,7 +687,7 @@ int tail_plan(int groups, int per_wave, int* nb) {
 }
 
 template <class SOL, int MX, int MBC, int AUXK, int NAUX, int TPB, int LIM>
-cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
+cudaError_t launch_one(const StepArgs& a, cudaStream_t st, int* bands) {
     constexpr int NX = MX + 2 * MBC;
     constexpr int PPB = TPB / NX;
     static_assert(PPB >= 1, "patch wider than the CTA");
@@ -732,9 +732,10 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
             StepArgs t = a;
             t.qsrc = a.qtail;
             t.nbands = best;
+            if (bands) *bands = best;
             t.band_first = 0;
             t.qtail = nullptr;
-            return launch_one<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(t, st);
+            return launch_one<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(t, st, nullptr);
         }
     } else if (a.nbands <= 1 && a.qtail && !a.desc && !a.treg && a.npatches > 0) {
         int tb = 1;
@@ -747,9 +748,10 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
             StepArgs t = a;
             t.qsrc = a.qtail;
             t.nbands = tb;
+            if (bands) *bands = tb;
             t.band_first = b0;
             t.qtail = nullptr;
-            return launch_one<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(t, st);
+            return launch_one<SOL, MX, MBC, AUXK, NAUX, TPB, LIM>(t, st, nullptr);
         }
     }
     const int nb = a.nbands > 1 ? a.nbands : 1;
@@ -773,54 +775,56 @@ cudaError_t launch_one(const StepArgs& a, cudaStream_t st) {
 // The Roe systems with order (2, 2) and the MC limiter on every wave (the
 // benchmarked configurations) get the method fixed at compile time.
 template <class SOL, int MX, int AUXK, int NAUX, int TPB>
-cudaError_t launch_lim(const StepArgs& a, cudaStream_t st) {
+cudaError_t launch_lim(const StepArgs& a, cudaStream_t st, int* bands) {
     if constexpr (SOL::M > 1) {
         bool mc = a.order0 == 2 && a.order1 == 2;
         for (int mw = 0; mw < SOL::W; ++mw) mc = mc && a.mthlim[mw] == 4;
-        if (mc) return launch_one<SOL, MX, 2, AUXK, NAUX, TPB, 4>(a, st);
+        if (mc) return launch_one<SOL, MX, 2, AUXK, NAUX, TPB, 4>(a, st, bands);
     }
-    return launch_one<SOL, MX, 2, AUXK, NAUX, TPB, 0>(a, st);
+    return launch_one<SOL, MX, 2, AUXK, NAUX, TPB, 0>(a, st, bands);
 }
 
 template <class SOL, int AUXK, int NAUX>
-cudaError_t launch_mx(int mx, int mbc, const StepArgs& a, cudaStream_t st) {
+cudaError_t launch_mx(int mx, int mbc, const StepArgs& a, cudaStream_t st, int* bands) {
     constexpr int TPB = SOL::M > 1 ? 256 : 128;
     if (mbc != 2) return cudaErrorInvalidValue;
     switch (mx) {
-        case 8: return launch_lim<SOL, 8, AUXK, NAUX, TPB>(a, st);
-        case 16: return launch_lim<SOL, 16, AUXK, NAUX, TPB>(a, st);
-        case 32: return launch_lim<SOL, 32, AUXK, NAUX, TPB>(a, st);
-        case 64: return launch_lim<SOL, 64, AUXK, NAUX, TPB>(a, st);
+        case 8: return launch_lim<SOL, 8, AUXK, NAUX, TPB>(a, st, bands);
+        case 16: return launch_lim<SOL, 16, AUXK, NAUX, TPB>(a, st, bands);
+        case 32: return launch_lim<SOL, 32, AUXK, NAUX, TPB>(a, st, bands);
+        case 64: return launch_lim<SOL, 64, AUXK, NAUX, TPB>(a, st, bands);
         default: return cudaErrorInvalidValue;
     }
 }
 
 }  // namespace
 
-// Returns cudaErrorInvalidValue for an unsupported (solver, mx, mbc, aux) combination.
+// Returns cudaErrorInvalidValue for an unsupported (solver, mx, mbc, aux) combination.  Where
+// the launcher split patches into row bands (and launched a copy of them first), *bands is
+// their number; it is left alone otherwise.
 cudaError_t launch_step(int solver, int aux_kind, int mwaves, int mx, int my, int mbc,
-                        const StepArgs& a, cudaStream_t st, int claw_version) {
+                        const StepArgs& a, cudaStream_t st, int claw_version, int* bands) {
     if (mx != my) return cudaErrorInvalidValue;
     // clawpack 5 exists in this form for the manifold advection solver only
     if (claw_version == 5 && solver != SOLVER_ADVECTION_MANIFOLD) return cudaErrorInvalidValue;
     switch (solver) {
         case SOLVER_ADVECTION:
             if (mwaves != 1) return cudaErrorInvalidValue;
-            if (aux_kind == AUX_SWIRL) return launch_mx<AdvectionSolver<1>, AUX_SWIRL, 2>(mx, mbc, a, st);
+            if (aux_kind == AUX_SWIRL) return launch_mx<AdvectionSolver<1>, AUX_SWIRL, 2>(mx, mbc, a, st, bands);
             if (aux_kind == AUX_STORED && a.maux >= 2)
-                return launch_mx<AdvectionSolver<1>, AUX_STORED, 2>(mx, mbc, a, st);
+                return launch_mx<AdvectionSolver<1>, AUX_STORED, 2>(mx, mbc, a, st, bands);
             return cudaErrorInvalidValue;
         case SOLVER_SWE_ROE:
             if (mwaves != 3 || aux_kind != AUX_NONE) return cudaErrorInvalidValue;
-            return launch_mx<SweRoeSolver, AUX_NONE, 0>(mx, mbc, a, st);
+            return launch_mx<SweRoeSolver, AUX_NONE, 0>(mx, mbc, a, st, bands);
         case SOLVER_EULER4_ROE:
             if (mwaves != 4 || aux_kind != AUX_NONE) return cudaErrorInvalidValue;
-            return launch_mx<Euler4RoeSolver, AUX_NONE, 0>(mx, mbc, a, st);
+            return launch_mx<Euler4RoeSolver, AUX_NONE, 0>(mx, mbc, a, st, bands);
         case SOLVER_ADVECTION_MANIFOLD:
             // capacity in aux(1), edge velocities in aux(2:3)
             if (mwaves != 1 || aux_kind != AUX_STORED || a.maux < 3) return cudaErrorInvalidValue;
-            if (claw_version == 5) return launch_mx<AdvectionManifoldSolver<1, true>, AUX_STORED, 3>(mx, mbc, a, st);
-            return launch_mx<AdvectionManifoldSolver<1>, AUX_STORED, 3>(mx, mbc, a, st);
+            if (claw_version == 5) return launch_mx<AdvectionManifoldSolver<1, true>, AUX_STORED, 3>(mx, mbc, a, st, bands);
+            return launch_mx<AdvectionManifoldSolver<1>, AUX_STORED, 3>(mx, mbc, a, st, bands);
         default: return cudaErrorInvalidValue;
     }
 }
