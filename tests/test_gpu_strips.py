@@ -68,6 +68,7 @@ def test_strips_equal_patches(gpu_lib, name, precision):
             cfl.append(s.advance_all_levels(t, dt))
             t += dt
         got.append((cfl, s.get_q()))
+        assert s.step_kernel_time(t, dt, 1)[1] == (fusion == 2)  # strips ran, patches ran
         s.close()
     (c1, q1), (c2, q2) = got
     if precision == 0:
@@ -78,7 +79,8 @@ def test_strips_equal_patches(gpu_lib, name, precision):
         assert np.max(np.abs(q1 - q2)) <= 3 * 64 * np.finfo(np.float32).eps * np.max(np.abs(q1))
 
 
-def test_strips_periodic_brick(gpu_lib):
+@pytest.mark.parametrize("precision", [0, 1])
+def test_strips_periodic_brick(gpu_lib, precision):
     """A periodic 2 x 2 brick (stored aux): the strip wraps around."""
     import forestclaw_b200 as fcb
     import oracle as O
@@ -87,7 +89,7 @@ def test_strips_periodic_brick(gpu_lib):
     got = []
     for fusion in (1, 2):
         o = cases.to_options(cfg)
-        o.ghost_fusion = fusion
+        o.ghost_fusion, o.precision = fusion, precision
         s = fcb.Solver(o)
         s.initialize()
         s.ghost_update(4, 4, 0.0, 0)  # level 3 of each block of the brick
@@ -95,5 +97,9 @@ def test_strips_periodic_brick(gpu_lib):
         for k in range(3):
             s.advance_all_levels(k * dt, dt)
         got.append(s.get_q())
+        assert s.step_kernel_time(0.0, dt, 1)[1] == (fusion == 2)
         s.close()
-    assert np.array_equal(got[0], got[1])
+    if precision == 0:
+        assert np.array_equal(got[0], got[1])
+    else:
+        assert np.max(np.abs(got[0] - got[1])) <= 3 * 64 * np.finfo(np.float32).eps * np.max(np.abs(got[0]))
