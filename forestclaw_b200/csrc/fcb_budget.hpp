@@ -5,15 +5,17 @@
 
 namespace fcb {
 
-// One owner's share of a total that all owners add to (any threads).
+// One owner's share, of at most `own` bytes, of a total of at most `cap` that all owners
+// add to (any threads).
 class KeptBytes {
   public:
-    KeptBytes(std::atomic<size_t>& total, size_t cap) : total_(total), cap_(cap) {}
+    KeptBytes(std::atomic<size_t>& total, size_t own, size_t cap) : total_(total), own_(own), cap_(cap) {}
     KeptBytes(const KeptBytes&) = delete;
     KeptBytes& operator=(const KeptBytes&) = delete;
     ~KeptBytes() { clear(); }
     // the owner keeps n bytes more, or may not
     bool add(size_t n) {
+        if (n > own_ - mine_) return false;
         size_t t = total_.load(std::memory_order_relaxed);
         do {
             if (n > cap_ || t > cap_ - n) return false;
@@ -28,7 +30,7 @@ class KeptBytes {
 
   private:
     std::atomic<size_t>& total_;
-    const size_t cap_;
+    const size_t own_, cap_;
     size_t mine_ = 0;
 };
 

@@ -868,8 +868,8 @@ Context::PlanWork& Context::plan_work(size_t k) {
     return *plan_work_[k];
 }
 
-// The contexts of a process keep at most 64 MB of build memory together (that of meshes
-// of about 20,000 patches).
+// A context keeps at most 64 MB of build memory (that of a mesh of about 20,000 patches),
+// the contexts of a process 512 MB together.
 std::atomic<size_t> Context::plan_bytes_{0};
 
 void Context::trim_plan_work() {

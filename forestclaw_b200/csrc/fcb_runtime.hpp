@@ -281,7 +281,7 @@ class Context {
     std::vector<std::tuple<int, int, int>> plan_todo_;
     std::vector<std::unique_ptr<PlanWork>> plan_work_;  // one per build that runs at once
     static std::atomic<size_t> plan_bytes_;  // kept by all contexts
-    KeptBytes plan_kept_{plan_bytes_, (size_t)64 << 20};
+    KeptBytes plan_kept_{plan_bytes_, (size_t)64 << 20, (size_t)512 << 20};
     std::vector<std::exception_ptr> plan_err_;
     std::vector<std::thread> plan_threads_;
     // pinned staging of the op and group buffers, and the event of its last upload
