@@ -33,6 +33,8 @@
 // one, their ghost cells read from the neighbours' interiors (fcb_strip.cuh).  B200,
 // mx = 16, us a step, unfused with its ghost fill -> fused: FP64 16,384 patches 149 -> 131,
 // 65,536 558 -> 500; mixed 136 -> 112, 475 -> 387.
+// The loops over components and waves (M = W = 1) are what is left of the form that also
+// served the systems; they vanish at compile time.
 // The kernel is a template on the compute type R of the Riemann solves,
 // limiters and transverse parts (SOL::Real): R = double is the FP64 form,
 // compiled without FMA contraction (fcb_step_pipe.cu); R = float is the mixed

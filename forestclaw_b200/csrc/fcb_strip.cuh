@@ -3,7 +3,7 @@
 //
 // Why strips: a patch of mx cells a side sweeps mx + 4 columns over mx + 7 rows (ghost
 // cells, pipeline), 1.8 cells of work per cell at mx = 16 and 2.8 at mx = 8; a strip of
-// 123 columns over 240 rows 1.07.  Swirl advection, level 8, mx = 16, one step on B200:
+// 121 columns over 241 rows 1.07.  Swirl advection, level 8, mx = 16, one step on B200:
 // FP64 0.508 ms with fused patches, 0.369 ms in strips with the same kernel (0.274 ms
 // with a kernel made for them, fcb_step_adv.cuh); mixed 0.375, 0.272 and 0.196 ms;
 // shallow water, 1024 x 1024 cells: 0.139 (mx = 32), 0.178 (16), 0.214 ms (8) in patches
