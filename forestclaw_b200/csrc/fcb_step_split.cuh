@@ -28,7 +28,9 @@
 // B200: 0.395 ms in the four-barrier form, 0.139 ms here (FP64 pipe 46 %, issue slots
 // 60 %; stalls: fixed latencies and the barrier); Euler, mx = 16, 4,096 patches: 0.856
 // and 0.320 ms; GeoClaw, mx = 32, 1,024 patches: 0.157 ms (pipelined form of one thread
-// per column: 0.57 ms).
+// per column: 0.57 ms).  Those are of states with a front's tail in many patches; after 20
+// steps of CFL 0.4 from the dam break, the quadrants and the lake: 0.119, 0.309 and 0.131 ms
+// (0.121, 0.339 and 0.133 with the Roe averages of out-of-range quotients formed from the states).
 //
 // Arithmetic, operation order and loop bounds are those of the reference
 // (src/solvers/fc2d_clawpack4.6/fortran_source/clawpack46_step2.f, clawpack46_flux2.f,
