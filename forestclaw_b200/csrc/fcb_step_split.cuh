@@ -29,8 +29,9 @@
 // 60 %; stalls: fixed latencies and the barrier); Euler, mx = 16, 4,096 patches: 0.856
 // and 0.320 ms; GeoClaw, mx = 32, 1,024 patches: 0.157 ms (pipelined form of one thread
 // per column: 0.57 ms).  Those are of states with a front's tail in many patches; after 20
-// steps of CFL 0.4 from the dam break, the quadrants and the lake: 0.119, 0.309 and 0.131 ms
-// (0.121, 0.339 and 0.133 with the Roe averages of out-of-range quotients formed from the states).
+// steps from the dam break and the lake (CFL 0.4) and the quadrants (0.2): 0.119, 0.131 and
+// 0.309 ms (0.121, 0.133 and 0.339 before the operators' path took the cells' quantities and
+// the range checks of dividends became one comparison).
 //
 // Arithmetic, operation order and loop bounds are those of the reference
 // (src/solvers/fc2d_clawpack4.6/fortran_source/clawpack46_step2.f, clawpack46_flux2.f,
