@@ -173,6 +173,7 @@ struct GhostArgs {
     const int32_t* groups; // group k = records [groups[k], groups[k+1]) (absolute indices into ops)
     int ngroups;
     int interp_fp32;       // mixed precision: coarse-to-fine interpolation in FP32
+    int sms;               // SMs of the device
     int wpg_log2;          // warps per group (log2), set by the launcher
 };
 

@@ -19,7 +19,6 @@
 #include <cuda_runtime.h>
 
 #include "fcb_device.h"
-#include "fcb_launch.hpp"
 
 namespace fcb {
 
@@ -326,12 +325,10 @@ void launch_ghost_shape(const GhostArgs& a, cudaStream_t st, int unroll, int blo
 
 cudaError_t launch_ghost_wave(const GhostArgs& a0, cudaStream_t st, int unroll) {
     if (a0.ngroups <= 0) return cudaSuccess;
-    int sms = 0;
-    if (const cudaError_t e = sm_count(&sms); e != cudaSuccess) return e;
     // warps per group (1 to 8): about 32 warps per SM
     GhostArgs a = a0;
     a.wpg_log2 = 0;
-    while (a.wpg_log2 < 3 && ((int64_t)a.ngroups << (a.wpg_log2 + 1)) <= sms * 32) ++a.wpg_log2;
+    while (a.wpg_log2 < 3 && ((int64_t)a.ngroups << (a.wpg_log2 + 1)) <= a.sms * 32) ++a.wpg_log2;
     const int blocks = (int)(((((int64_t)a.ngroups) << a.wpg_log2) * 32 + GHOST_TPB - 1) / GHOST_TPB);
     const int shape = (a.mbc == 2 && a.mx == a.my) ? a.mx : 0;
     switch (shape) {

@@ -60,15 +60,5 @@ cudaError_t per_device(PerDevice<N>& kept, int* out, const F& setup) {
     return e != cudaSuccess ? e : kept.get(dev, out, setup);
 }
 
-// SMs of the current device.
-inline cudaError_t sm_count(int* out) {
-    static PerDevice<> kept;
-    return per_device(kept, out, [](int* n) {
-        int dev = 0;
-        const cudaError_t e = cudaGetDevice(&dev);
-        return e != cudaSuccess ? e : cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev);
-    });
-}
-
 }  // namespace fcb
 #endif

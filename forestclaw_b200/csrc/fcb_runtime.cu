@@ -206,6 +206,9 @@ Context::Context(const fcb_options_t& o, cudaStream_t st, std::shared_ptr<Comm> 
 // The CFL words (first device use of a context: creation itself touches no device).
 void Context::ensure_scalars() {
     if (d_cfl_) return;
+    int dev = 0;
+    check(cudaGetDevice(&dev), "cudaGetDevice");
+    check(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev), "SM count");
     // [0] macro step, [1] level / batch, [2] global maximum, [3] autotuner,
     // [4] running maximum of the asynchronous macro steps, [5] fused macro step that is
     // waited for
@@ -1218,6 +1221,7 @@ void Context::run_plan(const GhostPlan& g) {
         a.groups = d_groups_.p + g.first_group + g.group_begin[w];  // group starts, then an end marker
         a.ngroups = g.group_begin[w + 1] - g.group_begin[w] - 1;
         a.interp_fp32 = opt_.precision == 1;
+        a.sms = sms_;
         check(launch_ghost_wave(a, st_, ghost_unroll_), "ghost wave");
         ++cnt_.count_ghost_waves;
         ++cnt_.count_kernel_launches;
@@ -2007,6 +2011,7 @@ int Context::tune_ghost_unroll(const GhostPlan& g) {
                 ga.groups = d_groups_.p + g.first_group + g.group_begin[w];
                 ga.ngroups = g.group_begin[w + 1] - g.group_begin[w] - 1;
                 ga.interp_fp32 = opt_.precision == 1;
+                ga.sms = sms_;
                 check(launch_ghost_wave(ga, st_, u), "tune ghost");
             }
         };

@@ -406,6 +406,7 @@ class Context {
     static constexpr int kCflLevel = 1, kCflFused = 5;  // words of d_cfl_ that only waited-for steps use
     unsigned long long* d_cfl_ = nullptr;  // (ensure_scalars lists the words)
     unsigned long long* h_cfl_ = nullptr;  // pinned readback of one CFL word
+    int sms_ = 0;                          // SMs of the context's device (ensure_scalars)
     unsigned cfl_zero_ = 0;                // bit i: word i (of those two) is zero already
     unsigned long long* zeroed_cfl(int i);
     double read_cfl(int i);                // copy CFL word [i] back, zero it and synchronize
